@@ -21,7 +21,9 @@ LIB = os.path.join(HERE, "libmaxlq_b200.so")
 SOURCES = ["engine.cu", "engine_f32.cu", "engine_f64.cu", "solver.cu", "capi.cu", "noalloc.cu", "diag.cu", "lsdev.cu",
            "ncdf.cpp", "kappa.cpp"]
 HEADERS = ["common.cuh", "fft.cuh", "kernels.cuh", "functors.cuh", "regfft.cuh", "cfft.cuh", "engine.cuh",
-           "engine_common.cuh", "engine_impl.cuh", "solver.cuh", "linesearch.cuh"]
+           "engine_common.cuh", "engine_impl.cuh", "engine_pass.cuh", "engine_pass.cu", "solver.cuh", "linesearch.cuh"]
+# the pass kernels: one object per precision and size with compile-time kernels, the slowest first
+PASS_UNITS = [(t, n) for n in (512, 256, 1024, 384, 768, 192, 128, 64, 96, 32, 48, 16) for t in ("float", "double")]
 # the device line search rounds every step as the host search does
 EXTRA_FLAGS = {"lsdev.cu": ["-fmad=false"]}
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -60,6 +62,11 @@ def build(force: bool = False, verbose: bool = False, ptxas_v: bool = False) -> 
     if ptxas_v:
         common += ["-Xptxas", "-v"]
     objs, cmds = [], []
+    for t, n in PASS_UNITS:
+        obj = os.path.join(objdir, f"engine_pass_{t}_{n}.o")
+        cmds.append(common + [f"-DMLQ_PASS_T={t}", f"-DMLQ_PASS_N={n}", "-c", os.path.join(CSRC, "engine_pass.cu"),
+                              "-o", obj])
+        objs.append(obj)
     for src in SOURCES:
         obj = os.path.join(objdir, os.path.splitext(src)[0] + ".o")
         cmds.append(common + EXTRA_FLAGS.get(src, []) + ["-c", os.path.join(CSRC, src), "-o", obj])

@@ -111,17 +111,34 @@ __device__ __forceinline__ cpx<T> cmul_s(cpx<T> a, cpx<T> w) {
 }
 
 // ----------------------------------------------------------------------------
-// Plan of a length-L transform held as E elements per thread: radix-E stages,
-// then one smaller power-of-two radix for the remainder.
+// Plan of a length-L transform held as E elements per thread.
+// L = 2^a: radix-E stages, then one smaller power-of-two radix for the
+// remainder.  L = 3 2^a, E = 3 2^e: the L/E = 2^(a-e) part first, in radix-2^e
+// stages and a smaller remainder, then one radix-E stage for the factor 3
+// (dft3m).  Every stage before the last then has a power-of-two stride, so
+// the twiddle index stays a mask and the threads of a line a power of two.
+// Against the run-time Stockham kernels (fft.cuh), which these sizes ran
+// before and which spend their time on FP64 twiddle loads and an integer
+// division per element: x inverse 986 -> 3800 GB/s, y forward 825 -> 3470, z
+// round trip 633 -> 1870 at 384^3 FP32, a CG iteration 58 -> 22 ms (mixed) and
+// at 192^3 7.8 -> 3.5 ms.  9 2^a would need a thread count of 3 2^j per line
+// and keeps the run-time kernels.
 // ----------------------------------------------------------------------------
 template <int L, int E>
 struct CPlan {
-    static_assert((L & (L - 1)) == 0 && (E & (E - 1)) == 0 && E >= 2 && E <= 16 && E <= L, "plan shape");
+    static constexpr bool THREE = L % 3 == 0;
+    static constexpr int L2 = THREE ? L / E : L;  // the part the leading stages transform
+    static constexpr int E2 = THREE ? E / 3 : E;  // and their radix
+    static_assert((L2 & (L2 - 1)) == 0 && (E2 & (E2 - 1)) == 0 && E2 >= 2 && E <= 24 && E <= L && L % E == 0 &&
+                      (!THREE || E % 3 == 0),
+                  "plan shape");
     static constexpr int TPL = L / E;
-    static constexpr int LGL = clog2(L), LGE = clog2(E);
+    static constexpr int LGL = clog2(L2), LGE = clog2(E2);
     static constexpr int NFULL = LGL / LGE, REMLG = LGL % LGE;
-    static constexpr int NST = NFULL + (REMLG ? 1 : 0);
-    __host__ __device__ static constexpr int radix(int s) { return s < NFULL ? E : (1 << REMLG); }
+    static constexpr int NST = NFULL + (REMLG ? 1 : 0) + (THREE ? 1 : 0);
+    __host__ __device__ static constexpr int radix(int s) {
+        return THREE && s == NST - 1 ? E : (s < NFULL ? E2 : (1 << REMLG));
+    }
     __host__ __device__ static constexpr int ns(int s) {
         int v = 1;
         for (int i = 0; i < s; ++i) v *= radix(i);
@@ -295,20 +312,31 @@ __device__ __forceinline__ void cfft(cpx<T> (&v)[E], int t, cpx<T>* sm, const Ma
 template <int N, typename T>
 struct CShape {
     static constexpr int L = N / 2;  // x lines: half-length complex transform
-    // x pass: elements per thread (a line stays within one warp)
-    static constexpr int EX = sizeof(T) == 4 ? (L >= 256 ? 16 : (L >= 64 ? 8 : 4)) : (L >= 512 ? 16 : (L >= 64 ? 8 : 4));
+    static constexpr bool THREE = N % 3 == 0;
+    // x pass: elements per thread (a line stays within one warp).  3 2^a: 12,
+    // the radix of the last stage (6 for the short L = 24, whose 4 threads
+    // then read whole 32-byte sectors).
+    static constexpr int EX = THREE ? (L >= 48 ? 12 : 6)
+                              : sizeof(T) == 4 ? (L >= 256 ? 16 : (L >= 64 ? 8 : 4))
+                                               : (L >= 512 ? 16 : (L >= 64 ? 8 : 4));
     static constexpr int TPLX = L / EX;
+    // threads per x block: 12 FP64 elements per thread would park more than
+    // an SM's shared memory in a six-output forward block of 256
+    static constexpr int XTHREADS = THREE && EX == 12 && sizeof(T) == 8 ? 128 : 256;
     // x pass twiddles: registers in FP32; a shared-memory table in FP64,
     // where the registers are needed for the data
     static constexpr bool XTW_REG = sizeof(T) == 4;
-    static constexpr int XLPB = 256 / TPLX;  // lines per x block
+    static constexpr int XLPB = XTHREADS / TPLX;  // lines per x block
     // row pitch: one pad element every EX; with two FP32 lines per warp the
     // second line's row starts half the banks away
     static constexpr int XPITCH = L + L / EX + (sizeof(T) == 4 && TPLX == 16 ? 8 : 0);
     static constexpr size_t XSMEM = ((size_t)XLPB * XPITCH + (XTW_REG ? 0 : L)) * sizeof(cpx<T>);
-    // y/z passes: tile rows of TX columns (64 or 128 bytes)
-    static constexpr int TX = sizeof(T) == 4 ? (N >= 512 ? 8 : 16) : (N >= 1024 ? 4 : 8);
-    static constexpr int EY = sizeof(T) == 4 ? (N >= 256 ? 16 : (N >= 128 ? 8 : 4)) : (N >= 1024 ? 16 : (N >= 128 ? 8 : 4));
+    // y/z passes: tile rows of TX columns (64 or 128 bytes; 8 columns in FP32
+    // for 3 2^a, where nx = N/3 + 1 leaves a wider last tile mostly empty)
+    static constexpr int TX = sizeof(T) == 4 ? (N >= 512 || N == 16 || THREE ? 8 : 16) : (N >= 768 ? 4 : 8);
+    static constexpr int EY = THREE ? (N >= 768 && sizeof(T) == 4 ? 24 : 12)
+                              : sizeof(T) == 4 ? (N >= 256 ? 16 : (N >= 128 ? 8 : 4))
+                                               : (N >= 1024 ? 16 : (N >= 128 ? 8 : 4));
     static constexpr int TPLY = N / EY;
     static constexpr int YTHREADS = TX * TPLY;
     static_assert(TPLX <= 32 && 32 % TPLX == 0, "x line within a warp");
@@ -337,7 +365,10 @@ struct YShape {
     static constexpr bool PAIR = V == 8 || V == 9;
     static constexpr int PAIR_MINB = V == 9 ? 3 : 2;
     static constexpr int VB = (CW || MB3) ? 0 : (V >= 3 ? V - 3 : V);
-    static constexpr int EY = CW ? N / 32 : (VB == 0 ? CShape<N, T>::EY : (VB == 1 ? (F32 ? 8 : 16) : (F32 ? 16 : 8)));
+    static constexpr bool THREE = N % 3 == 0;  // 3 2^a: V = 0, 1 (24 elements), 2 (the other tile width) and 8
+    static constexpr int EY = CW      ? (N >= 32 ? N / 32 : 1)
+                              : THREE ? (VB == 1 ? 24 : CShape<N, T>::EY)
+                                      : (VB == 0 ? CShape<N, T>::EY : (VB == 1 ? (F32 ? 8 : 16) : (F32 ? 16 : 8)));
     static constexpr int TX = CW ? (V == 5 ? (F32 ? 8 : 4) : (F32 ? 16 : 2))
                                  : (VB == 0 ? CShape<N, T>::TX : (VB == 1 ? 8 : (F32 ? 16 : 4)));
     static constexpr bool TWREG = V == 3 || V == 4;
@@ -362,7 +393,10 @@ struct YShape {
     static constexpr int YMINB = CW ? (CW_MINB < 1 ? 1 : CW_MINB)
                                     : MB3 ? 3 : (TWREG ? 1 : (YTHREADS <= 256 ? 2 : (F32 && EY <= 8 ? 2 : 1)));
     static constexpr bool valid =
-        V == 0 || (PAIR ? (F32 && N >= 256 && N <= (V == 9 ? 512 : 1024)) :
+        V == 0 || (THREE ? (N >= 192 && ZSMEM <= 200 * 1024 &&
+                            ((V == 8 && F32) || (V == 1 && F32 && EY != CShape<N, T>::EY) ||
+                             (V == 2 && YTHREADS % 32 == 0 && TX != CShape<N, T>::TX))) :
+        PAIR ? (F32 && N >= 256 && N <= (V == 9 ? 512 : 1024)) :
         (MB3 ? (N >= 256 && YTHREADS <= 256 && 3 * (ZSMEM + 1024) <= 228 * 1024) :
          CW ? (N >= 256 && EY >= 2 && EY <= 16 && YTHREADS % 32 == 0 && YTHREADS <= 512 && ZSMEM <= 227 * 1024)
             : (N >= 256 && TPLY >= 2 && YTHREADS % 32 == 0 && YTHREADS <= 512 && ZSMEM <= 200 * 1024 &&
@@ -418,11 +452,11 @@ __device__ __forceinline__ void block_reduce_to(const double* acc, double* out) 
 }
 
 // ----------------------------------------------------------------------------
-// x stage, inverse (c2r).  grid = (G, narr), block = 256.  Each block walks
-// groups of 256/TPL lines of array blockIdx.y.
+// x stage, inverse (c2r).  grid = (G, narr), block = XTHREADS.  Each block
+// walks groups of XTHREADS/TPL lines of array blockIdx.y.
 // ----------------------------------------------------------------------------
 template <int N, typename T>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(CShape<N, T>::XTHREADS, 512 / CShape<N, T>::XTHREADS)
     xinv_c_kernel(XInvArgs<T> a, const cpx<T>* __restrict__ twL, const cpx<T>* __restrict__ twN) {
     using S = CShape<N, T>;
     constexpr int L = S::L, E = S::EX, TPL = S::TPLX, LPB = S::XLPB, PITCH = S::XPITCH;
@@ -486,8 +520,8 @@ __global__ void __launch_bounds__(256, 2)
 // ----------------------------------------------------------------------------
 // x stage, forward: functor on the physical inputs, then the real FFT of each
 // functor output along x (a complex transform of length N/2 of the packed
-// pairs, then the half-spectrum split).  grid = G, block = 256: each block
-// walks groups of 256/TPL lines; output 0 stays in registers, outputs 1.. are
+// pairs, then the half-spectrum split).  grid = G, block = XTHREADS: each
+// block walks groups of XTHREADS/TPL lines; output 0 stays in registers, outputs 1.. are
 // parked in thread-private shared-memory slots until their turn.
 // ----------------------------------------------------------------------------
 template <int N, typename T, int NOUT>
@@ -497,10 +531,12 @@ struct XFwdSmem {
     static constexpr size_t BYTES = (STAGE + (size_t)S::XLPB * S::XPITCH + (S::XTW_REG ? 0 : S::L)) * sizeof(cpx<T>);
 };
 
-// positions whose inputs are loaded together: about 32 loads per thread
+// positions whose inputs are loaded together: about 32 loads per thread (a
+// divisor of the e positions)
 __host__ __device__ constexpr int xfwd_chunk(int nin, int e) {
     int c = 1;
-    while (2 * c <= e && 2 * c * nin <= 32) c *= 2;
+    for (int d = 2; d <= e; ++d)
+        if (e % d == 0 && d * nin <= 32) c = d;
     return c;
 }
 
@@ -511,7 +547,7 @@ constexpr int xfwd_minb() {
 }
 
 template <int N, typename T, class F>
-__global__ void __launch_bounds__(256, xfwd_minb<F>())
+__global__ void __launch_bounds__(CShape<N, T>::XTHREADS, xfwd_minb<F>() * 256 / CShape<N, T>::XTHREADS)
     xfwd_c_kernel(XFwdArgs<T> a, F f, const cpx<T>* __restrict__ twL, const cpx<T>* __restrict__ twN) {
     using S = CShape<N, T>;
     constexpr int NIN = F::NIN, NOUT = F::NOUT, NR = F::NRED;
@@ -1207,7 +1243,7 @@ __global__ void __launch_bounds__(YShape<N, T, V>::YTHREADS, YShape<N, T, V>::YM
 // ----------------------------------------------------------------------------
 template <int N>
 struct PairShape {
-    static constexpr int E = 8, NP = 4;
+    static constexpr int E = N % 3 == 0 ? 12 : 8, NP = 4;
     static constexpr int TPL = N / E;         // threads per column pair
     static constexpr int THREADS = NP * TPL;
     static constexpr int TILE = N * NP;       // float4 slots of one tile

@@ -518,7 +518,7 @@ class Engine : public EngineBase {
     bool reg_ok_ = false;
     cpx<T>* d_twT_ = nullptr;  // twiddle pool in T
     RPlan rplan(int L) const;
-    // kernels specialised at compile time for n in {64, ..., 1024} (cfft.cuh)
+    // kernels specialised at compile time for n of dispatch_n (cfft.cuh)
     bool cfft_ok_ = false;
     int persistent_blocks(const void* kernel, int threads, size_t smem);
     std::map<const void*, int> occ_;
@@ -553,6 +553,8 @@ class Engine : public EngineBase {
     void zfwd_c(ZFwdArgs<T>& za, int narr);
     template <int NN>
     void zinv_c(ZInvArgs<T>& za, int narr);
+    template <int NN>
+    void zinv_multi_c(ZInvMultiArgs<T>& za, int nops);
     int reg_tx() const;
     int reg_lx(int nrows_per_line, size_t pitch) const;
     // pass launchers (register kernels when reg_ok_, shared-memory Stockham otherwise)

@@ -58,10 +58,18 @@ static void allow_smem(K kernel) {
     }
 }
 
-// f(std::integral_constant<int, n>) for the sizes with compile-time kernels
+// f(std::integral_constant<int, n>) for the sizes with compile-time kernels:
+// 2^a and 3 2^a from 16 to 1024 (24 would leave one thread per x line)
 template <class Fn>
 static bool dispatch_n(int n, Fn&& f) {
     switch (n) {
+        case 16: f(std::integral_constant<int, 16>{}); return true;
+        case 32: f(std::integral_constant<int, 32>{}); return true;
+        case 48: f(std::integral_constant<int, 48>{}); return true;
+        case 96: f(std::integral_constant<int, 96>{}); return true;
+        case 192: f(std::integral_constant<int, 192>{}); return true;
+        case 384: f(std::integral_constant<int, 384>{}); return true;
+        case 768: f(std::integral_constant<int, 768>{}); return true;
         case 64: f(std::integral_constant<int, 64>{}); return true;
         case 128: f(std::integral_constant<int, 128>{}); return true;
         case 256: f(std::integral_constant<int, 256>{}); return true;

@@ -25,7 +25,7 @@ Engine<T>::Engine(const mlq_params& p) : EngineBase(p) {
     widen(P.q / 2.0);
     if (!use_e_u) widen(P.q - 4.0);
     reg_ok_ = n >= 64 && (n & (n - 1)) == 0;
-    cfft_ok_ = reg_ok_ && n <= 1024;
+    cfft_ok_ = dispatch_n(n, [](auto) {});
     if (const char* kv = std::getenv("MLQ_PASS_KERNELS")) cfft_ok_ = cfft_ok_ && std::string(kv) != "reg";
     pitch_even_ = cfft_ok_ && sizeof(T) == 4;
     // the mixed path keeps its CG state (every state vector's Fourier
@@ -57,8 +57,9 @@ Engine<T>::Engine(const mlq_params& p) : EngineBase(p) {
     tune_yz();
     // z-slab streaming when the physical fields the programs keep resident
     // (up to ~72 with the line-search setup) would not fit in free memory;
-    // MLQ_SLAB_PLANES=k forces k planes per slab (0: never)
-    if (cfft_ok_) {
+    // MLQ_SLAB_PLANES=k forces k planes per slab (0: never).  A slab is a power
+    // of two planes of whole x blocks: n = 2^a >= 64.
+    if (cfft_ok_ && reg_ok_) {
         int want = -1;
         if (const char* e = std::getenv("MLQ_SLAB_PLANES")) {
             want = std::atoi(e) > 0 ? std::atoi(e) : -1;
@@ -140,10 +141,10 @@ void Engine<T>::xinv_c(XInvArgs<T>& xa, int narr) {
     const size_t smem = S::XSMEM;
     auto kern = xinv_c_kernel<NN, T>;
     allow_smem(kern);
-    const int G = persistent_blocks((const void*)kern, 256, smem);
+    const int G = persistent_blocks((const void*)kern, S::XTHREADS, smem);
     const long ng = xa.nlines / LPB;
     dim3 grid((unsigned)std::min<long>(ng, std::max(1, G / narr)), narr);
-    kern<<<grid, 256, smem, stream>>>(xa, d_twT_ + tw_off.at(NN / 2), d_twT_ + tw_off.at(NN));
+    kern<<<grid, S::XTHREADS, smem, stream>>>(xa, d_twT_ + tw_off.at(NN / 2), d_twT_ + tw_off.at(NN));
 }
 
 // y/z launches of tile-shape variant V (cfft.cuh YShape)
@@ -535,13 +536,13 @@ void Engine<T>::xfwd_c(XFwdArgs<T>& xa, const F& f) {
     const size_t smem = XFwdSmem<NN, T, F::NOUT>::BYTES;
     auto kern = xfwd_c_kernel<NN, T, F>;
     allow_smem(kern);
-    const int G = persistent_blocks((const void*)kern, 256, smem);
+    const int G = persistent_blocks((const void*)kern, S::XTHREADS, smem);
     const long ng = xa.nlines / S::XLPB;
     const int grid = (int)std::min<long>(ng, G);
     last_xblocks_ = grid;
     if (F::NRED > 0) ensure_partials((long)grid * F::NRED);
     xa.partials = d_partials;
-    kern<<<grid, 256, smem, stream>>>(xa, f, d_twT_ + tw_off.at(NN / 2), d_twT_ + tw_off.at(NN));
+    kern<<<grid, S::XTHREADS, smem, stream>>>(xa, f, d_twT_ + tw_off.at(NN / 2), d_twT_ + tw_off.at(NN));
 }
 
 template <typename T>
@@ -762,10 +763,15 @@ void Engine<T>::launch_zinv_multi(ZInvMultiArgs<T>& za, int nops, const Band& b,
     cudaEvent_t ev = prof_mark();
     dispatch_n(n, [&](auto nc) {
         constexpr int NN = decltype(nc)::value;
-        this->template with_variant<NN>(
-            YV_ZINV, [&](auto vc) { this->template zinv_multi_cv<NN, decltype(vc)::value>(za, nops); });
+        this->template zinv_multi_c<NN>(za, nops);
     });
     launched("z_inv", zbytes, ev);
+}
+
+template <typename T>
+template <int NN>
+void Engine<T>::zinv_multi_c(ZInvMultiArgs<T>& za, int nops) {
+    with_variant<NN>(YV_ZINV, [&](auto vc) { this->template zinv_multi_cv<NN, decltype(vc)::value>(za, nops); });
 }
 
 template <typename T>

@@ -113,13 +113,43 @@ __device__ __forceinline__ void dft16(cpx<T>* v) {
     }
 }
 
+// radix 3 M (M = 2, 4, 8) as 3 x M by the prime-factor (Good-Thomas) index
+// maps, which need no twiddles between the two factors: with the input at
+// n = (M n1 + 3 n2) mod 3M and the output at k = 3 (3^-1 mod M) k2 +
+// M (M^-1 mod 3) k1 mod 3M, W_3M^(n k) = W_3^(n1 k1) W_M^(n2 k2).
+template <int M, int SIGN, typename T>
+__device__ __forceinline__ void dft3m(cpx<T>* v) {
+    constexpr int R = 3 * M;
+    constexpr int IM = M == 4 ? 1 : 2;              // M^-1 mod 3
+    constexpr int I3 = M == 2 ? 1 : 3;              // 3^-1 mod M
+    cpx<T> a[3][M];
+#pragma unroll
+    for (int n1 = 0; n1 < 3; ++n1) {
+#pragma unroll
+        for (int n2 = 0; n2 < M; ++n2) a[n1][n2] = v[(M * n1 + 3 * n2) % R];
+        if (M == 2) dft2<SIGN>(a[n1]);
+        if (M == 4) dft4v<SIGN>(a[n1]);
+        if (M == 8) dft8<SIGN>(a[n1]);
+    }
+#pragma unroll
+    for (int k2 = 0; k2 < M; ++k2) {
+        cpx<T> b[3] = {a[0][k2], a[1][k2], a[2][k2]};
+        dft3<SIGN>(b);
+#pragma unroll
+        for (int k1 = 0; k1 < 3; ++k1) v[(M * IM * k1 + 3 * I3 * k2) % R] = b[k1];
+    }
+}
+
 template <int R, int SIGN, typename T>
 __device__ __forceinline__ void dftR(cpx<T>* v) {
-    if (R == 2) dft2<SIGN>(v);
-    if (R == 3) dft3<SIGN>(v);
-    if (R == 4) dft4v<SIGN>(v);
-    if (R == 8) dft8<SIGN>(v);
-    if (R == 16) dft16<SIGN>(v);
+    if constexpr (R == 2) dft2<SIGN>(v);
+    if constexpr (R == 3) dft3<SIGN>(v);
+    if constexpr (R == 4) dft4v<SIGN>(v);
+    if constexpr (R == 6) dft3m<2, SIGN>(v);
+    if constexpr (R == 8) dft8<SIGN>(v);
+    if constexpr (R == 12) dft3m<4, SIGN>(v);
+    if constexpr (R == 16) dft16<SIGN>(v);
+    if constexpr (R == 24) dft3m<8, SIGN>(v);
 }
 
 // One Stockham stage of radix R over all lines.
