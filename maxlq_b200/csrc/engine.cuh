@@ -431,6 +431,24 @@ class Engine : public EngineBase {
     // tau0: the previous step, whose neighbourhood the trials visit (<= 0: none)
     void ls_setup(const SVec* u, const SVec* d, double tau0 = 0.0);
     void ls_trial(double tau, double out[3], double* lqq);
+    // the same at the other exponents (and on the e_u branch): the setup
+    // forms what is quadratic in tau, a trial transforms the products that
+    // are not.  Resident mode only; MLQ_REUSE=0 evaluates R whole per trial.
+    bool lsg_ok() const { return !ls_ok() && !slab_ && reuse_on_; }
+    bool lsg_fits();
+    void lsg_setup(const SVec* u, const SVec* d, double tau0 = 0.0);
+    void lsg_trial(double tau, double out[3], double* lqq);
+    int lsg_power_sq(double k);
+    std::vector<int> lsg_ud_;  // physical fields of u and d in this line search
+    // parts of the setups
+    struct LsFields {
+        std::vector<int> ud, all, grads;  // u, d; u, Du, d, Dd; Du, Dd
+    };
+    LsFields ls_fields(const SVec* u, const SVec* d);
+    void ls_w_fields(const LsFields& lf);
+    void ls_qg_fields(const LsFields& lf, bool g_phys);
+    void ls_dev_alloc();
+    void ls_interval_dev(double tau0);
     // Where S(tau) = S0 + tau S1 + tau^2 S2 (the dealiased |phi|^2) is >= 0 at
     // every point, the clamp of calc_uk is inactive and P2(g^2) = S(tau): a
     // trial in [ls_c_.tlo, ls_c_.thi] is then a polynomial in tau of the
@@ -570,6 +588,7 @@ class Engine : public EngineBase {
     // |u|^k chain (calc_uk); memoised per program
     std::map<double, PowField> memo_;
     int tmp_next_ = 0, spec_next_ = 0;
+    int ps_ = 18, pa_ = 19;  // physical fields of the S and A that the chain reads (PS, PA)
     void chain_reset() {
         memo_.clear();
         tmp_next_ = 0;

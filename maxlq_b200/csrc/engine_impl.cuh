@@ -1459,6 +1459,18 @@ enum : int {
     WLQ = 46,   // work spectra: -Lap^-1 P2(Q_a) (3), read by the next gradient
     WS = 49,    // work spectrum of S = P2(|u|^2) (gradient program, transport)
 };
+// the line search at other exponents: besides the fields above, the trial's
+// S(tau) and A(tau), G_a = P2 coefficients of |grad phi|^2 in physical space,
+// and on the e_u branch the raw W_aj (3a+j) and E_j
+enum : int {
+    LTS = 110,
+    LTA = 111,
+    LG = 112,   // 112..114
+    LW = 115,   // 115..123
+    LE = 124,   // 124..126
+    LEND = 127,
+    WTA2 = 54,  // work spectrum of |phi|^{q-2} (e_u branch)
+};
 }  // namespace
 
 // the physical-field memo covers u, grad u (0..11), S and A (18, 19) and the
@@ -1582,7 +1594,7 @@ PowField Engine<T>::chain(double k) {
         FGPow fp;
         fp.k = k;
         fp.thresh = 1;
-        pointwise(fp, {PS}, {f.phys});
+        pointwise(fp, {ps_}, {f.phys});
     } else if (k + MACH_EPSILON < 2.0) {
         const int c = band_cut_for_order(n, k);
         if (c >= n / 2) {
@@ -1594,7 +1606,7 @@ PowField Engine<T>::chain(double k) {
                 FGPow fp;
                 fp.k = k;
                 fp.thresh = 0;
-                pointwise(fp, {PS}, {f.phys});
+                pointwise(fp, {ps_}, {f.phys});
             }
         } else {
             const Band bk = make_band(c);
@@ -1610,13 +1622,13 @@ PowField Engine<T>::chain(double k) {
                 o.spec = wspec(f.spec);
                 o.spec_f64 = wf64<T>();
             }
-            fwd(bk, fp, {PS}, {o});
+            fwd(bk, fp, {ps_}, {o});
         }
     } else {
         PowField prev = chain(k - 2.0);
         f.kind = PowField::BAND;
         if (prev.kind == PowField::ONE) {
-            f.phys = PA;
+            f.phys = pa_;
             f.spec = WA;
         } else {
             ensure_phys(prev);
@@ -1626,7 +1638,7 @@ PowField Engine<T>::chain(double k) {
             o.phys_out = f.phys;
             o.spec = wspec(f.spec);
             o.spec_f64 = wf64<T>();
-            fwd(b2, FMul{}, {PA, prev.phys}, {o});
+            fwd(b2, FMul{}, {pa_, prev.phys}, {o});
         }
     }
     memo_[k] = f;
@@ -2234,7 +2246,7 @@ double Engine<T>::transport_pieces(const SVec* u, const SVec* d, double tau, con
         inv(b2, io);
     }
     const PhysMemo m = pm_;  // this program's own writes below keep it
-    if (memo && q == 4.0 && !use_e_u && ls_clamp_free(tau)) {
+    if (memo && ls_clamp_free(tau)) {
         // |w|^2 = S_0 + tau S_1 + tau^2 S_2 (the line search's coefficient
         // fields, P2 linear) is >= 0 at every point, so A = P2(max(S, 0)) = S
         FPolyS f;
@@ -2422,15 +2434,12 @@ __global__ void __launch_bounds__(RED_THREADS)
     }
 }
 
+// The fields of a line search along phi = u + tau d that every exponent uses:
+// u, d and their gradients, the coefficients of P2(|phi|^2), and the memo of
+// them for the transport and the next gradient.
 template <typename T>
-void Engine<T>::ls_setup(const SVec* u, const SVec* d, double tau0) {
-    const long nc = spec_ncomp();
-    ls_free_val_ = -1;
-    ls_dev_ = ls_device_ready();
-    if (ls_dev_ && !d_ls_) {
-        d_ls_ = (LsDevState*)dev_alloc(sizeof(LsDevState));
-        MLQ_CUDA(cudaMallocHost(&h_ls_, 1024));
-    }
+typename Engine<T>::LsFields Engine<T>::ls_fields(const SVec* u, const SVec* d) {
+    LsFields lf;
     // u and grad u are still in PU, PD when the gradient program of this
     // iteration transformed the same spectrum
     const bool reuse_u = !slab_ && reuse_on_ && pu_of_ == (const void*)u;
@@ -2456,39 +2465,40 @@ void Engine<T>::ls_setup(const SVec* u, const SVec* d, double tau0) {
         pm_.idu = idu;
         pm_.ls = true;
     }
-    std::vector<int> ud = {iu, iu + 1, iu + 2, LD, LD + 1, LD + 2};
-    std::vector<int> all;
-    for (int i = 0; i < 3; ++i) all.push_back(iu + i);
-    for (int i = 0; i < 9; ++i) all.push_back(idu + i);
-    for (int i = 0; i < 3; ++i) all.push_back(LD + i);
-    for (int i = 0; i < 9; ++i) all.push_back(LDD + i);
-    std::vector<int> grads;
-    for (int i = 0; i < 9; ++i) grads.push_back(idu + i);
-    for (int i = 0; i < 9; ++i) grads.push_back(LDD + i);
+    lf.ud = {iu, iu + 1, iu + 2, LD, LD + 1, LD + 2};
+    for (int i = 0; i < 3; ++i) lf.all.push_back(iu + i);
+    for (int i = 0; i < 9; ++i) lf.all.push_back(idu + i);
+    for (int i = 0; i < 3; ++i) lf.all.push_back(LD + i);
+    for (int i = 0; i < 9; ++i) lf.all.push_back(LDD + i);
+    for (int i = 0; i < 9; ++i) lf.grads.push_back(idu + i);
+    for (int i = 0; i < 9; ++i) lf.grads.push_back(LDD + i);
     // P2 of the coefficients of |phi|^2 (calc_uk 2332-2333).  The tau^0 one,
     // P2(|u|^2), is the gradient program's S when it ran for this u.
-    {
-        const bool s0 = !slab_ && reuse_on_ && ws_of_ == (const void*)u;
-        ls_p0_ = s0 ? (int)PS : (int)LS;
-        ls_w0_ = s0 ? WS : WLS;
-        FwdOut o[3];
-        for (int a = 0; a < 3; ++a) {
-            o[a].phys_out = LS + a;
-            o[a].spec = wspec(WLS + a);
-            o[a].spec_f64 = wf64<T>();
-        }
-        if (s0)
-            fwd(b2, FLSS12{}, ud, {o[1], o[2]});
-        else
-            fwd(b2, FLSS{}, ud, {o[0], o[1], o[2]});
+    const bool s0 = !slab_ && reuse_on_ && ws_of_ == (const void*)u;
+    ls_p0_ = s0 ? (int)PS : (int)LS;
+    ls_w0_ = s0 ? WS : WLS;
+    FwdOut o[3];
+    for (int a = 0; a < 3; ++a) {
+        o[a].phys_out = LS + a;
+        o[a].spec = wspec(WLS + a);
+        o[a].spec_f64 = wf64<T>();
     }
-    // P2 of the coefficients of W_j = sum_i phi_i d_j phi_i (calc_vgraduvgradu /
-    // calc_vvgradu, v = phi).  W_j = (1/2) d_j |phi|^2, and when the cut c
-    // satisfies 3c < N the dealiased grid product of two band-limited fields
-    // is the band truncation of their exact product (its aliases land beyond
-    // the cut), so P2(W_j) = (1/2) d_j P2(|phi|^2): the derivatives of the
-    // S_a spectra just formed.  For 3c >= N (N divisible by 3) the products
-    // are formed and dealiased as the reference does.
+    if (s0)
+        fwd(b2, FLSS12{}, lf.ud, {o[1], o[2]});
+    else
+        fwd(b2, FLSS{}, lf.ud, {o[0], o[1], o[2]});
+    return lf;
+}
+
+// P2 of the coefficients of W_j = sum_i phi_i d_j phi_i (calc_vgraduvgradu /
+// calc_vvgradu, v = phi).  W_j = (1/2) d_j |phi|^2, and when the cut c
+// satisfies 3c < N the dealiased grid product of two band-limited fields
+// is the band truncation of their exact product (its aliases land beyond
+// the cut), so P2(W_j) = (1/2) d_j P2(|phi|^2): the derivatives of the
+// S_a spectra just formed.  For 3c >= N (N divisible by 3) the products
+// are formed and dealiased as the reference does.
+template <typename T>
+void Engine<T>::ls_w_fields(const LsFields& lf) {
     if (reuse_on_ && 3 * b2.cut < n) {
         std::vector<InvOut> g;
         for (int a = 0; a < 3; ++a)
@@ -2501,30 +2511,73 @@ void Engine<T>::ls_setup(const SVec* u, const SVec* d, double tau0) {
             }
         inv(b2, g);
     } else {
-        std::vector<int> uself(all.begin(), all.begin() + 12), dself(all.begin() + 12, all.end());
+        std::vector<int> uself(lf.all.begin(), lf.all.begin() + 12), dself(lf.all.begin() + 12, lf.all.end());
         FwdOut o[3];
         for (int j = 0; j < 3; ++j) o[j].phys_out = LV + j;
         fwd(b2, FLSW<0>{}, uself, {o[0], o[1], o[2]});
         for (int j = 0; j < 3; ++j) o[j].phys_out = LV + 3 + j;
-        fwd(b2, FLSW<1>{}, all, {o[0], o[1], o[2]});
+        fwd(b2, FLSW<1>{}, lf.all, {o[0], o[1], o[2]});
         for (int j = 0; j < 3; ++j) o[j].phys_out = LV + 6 + j;
         fwd(b2, FLSW<0>{}, dself, {o[0], o[1], o[2]});
     }
-    // p_a = -Lap^-1 P2(Q_a) and the spectra of P2(|grad phi|^2)_a
-    {
-        FwdOut o[6];
-        for (int a = 0; a < 3; ++a) {
-            o[a].sym = SYM_INV_KSQ;
-            o[a].phys_out = LP + a;
-            if (!slab_) {  // the next gradient's pressure source is a polynomial in tau of these
-                o[a].spec = wspec(WLQ + a);
-                o[a].spec_f64 = wf64<T>();
-            }
+}
+
+// p_a = -Lap^-1 P2(Q_a) and the spectra of P2(|grad phi|^2)_a (or, with
+// g_phys, these fields in physical space)
+template <typename T>
+void Engine<T>::ls_qg_fields(const LsFields& lf, bool g_phys) {
+    FwdOut o[6];
+    for (int a = 0; a < 3; ++a) {
+        o[a].sym = SYM_INV_KSQ;
+        o[a].phys_out = LP + a;
+        if (!slab_) {  // the next gradient's pressure source is a polynomial in tau of these
+            o[a].spec = wspec(WLQ + a);
+            o[a].spec_f64 = wf64<T>();
+        }
+        if (g_phys) {
+            o[3 + a].phys_out = LG + a;
+        } else {
             o[3 + a].spec = wspec(WLG + a);
             o[3 + a].spec_f64 = wf64<T>();
         }
-        fwd(b2, FLSQG{}, grads, {o[0], o[1], o[2], o[3], o[4], o[5]});
     }
+    fwd(b2, FLSQG{}, lf.grads, {o[0], o[1], o[2], o[3], o[4], o[5]});
+}
+
+// the line search's state on the device, and its pinned host side
+template <typename T>
+void Engine<T>::ls_dev_alloc() {
+    if (d_ls_) return;
+    d_ls_ = (LsDevState*)dev_alloc(sizeof(LsDevState));
+    MLQ_CUDA(cudaMallocHost(&h_ls_, 1024));
+}
+
+// clamp-free intervals of S(tau) and the polynomial coefficients, left on
+// the device (d_ls_->poly)
+template <typename T>
+void Engine<T>::ls_interval_dev(double tau0) {
+    LsAnchorSet an;
+    ls_anchors(tau0, an.a);
+    const int grid = grid_for(n3, RED_THREADS, 148 * 4);
+    ensure_partials((long)grid * 2 * (LS_ANCHORS + 1));
+    cudaEvent_t ev = prof_mark();
+    ls_interval_kernel<T><<<grid, RED_THREADS, 0, stream>>>(phys(ls_phys(0)), phys(ls_phys(1)), phys(ls_phys(2)), n3,
+                                                            an, d_partials);
+    launched("ls_interval", 3.0 * n3 * sizeof(T), ev);
+    ls_launch_coef(d_ls_, d_results, d_partials, grid, an, stream);
+    launched();
+    ls_host_poly_ = false;
+}
+
+template <typename T>
+void Engine<T>::ls_setup(const SVec* u, const SVec* d, double tau0) {
+    ls_free_val_ = -1;
+    ls_dev_ = ls_device_ready();
+    if (ls_dev_) ls_dev_alloc();
+    const LsFields lf = ls_fields(u, d);
+    const std::vector<int>& ud = lf.ud;
+    ls_w_fields(lf);
+    ls_qg_fields(lf, false);
     // R2 and R3 integrands as polynomials in tau
     std::vector<int> rin;
     for (int i = 0; i < 9; ++i) rin.push_back(LV + i);
@@ -2549,22 +2602,13 @@ void Engine<T>::ls_setup(const SVec* u, const SVec* d, double tau0) {
         sdots(*this, p3, 152);
     }
     // the interval of tau around 0 on which S(tau) >= 0 everywhere
+    if (ls_dev_) {  // on the device, with the coefficients: no host round trip
+        ls_interval_dev(tau0);
+        return;
+    }
     LsAnchorSet an;
     ls_anchors(tau0, an.a);
     constexpr int W = 2 * (LS_ANCHORS + 1);  // interval ends per block
-    if (ls_dev_) {
-        // on the device, with the coefficients: no host round trip
-        const int grid = grid_for(n3, RED_THREADS, 148 * 4);
-        ensure_partials((long)grid * W);
-        cudaEvent_t ev = prof_mark();
-        ls_interval_kernel<T><<<grid, RED_THREADS, 0, stream>>>(phys(ls_phys(0)), phys(ls_phys(1)),
-                                                                phys(ls_phys(2)), n3, an, d_partials);
-        launched("ls_interval", 3.0 * n3 * sizeof(T), ev);
-        ls_launch_coef(d_ls_, d_results, d_partials, grid, an, stream);
-        launched();
-        ls_host_poly_ = false;
-        return;
-    }
     double lo[LS_ANCHORS + 1], hi[LS_ANCHORS + 1];
     for (int k = 0; k <= LS_ANCHORS; ++k) {
         lo[k] = -1e300;
@@ -2839,6 +2883,193 @@ void Engine<T>::ls_trial(double tau, double out[3], double* lqq) {
     fetch_results();
     ls_fft_R(ls_c_, q, cv, cp, h_results + 130, tau, out, &l);
     if (lqq) *lqq = l;
+}
+
+// ----------------------------------------------------------------------------
+// line search along phi = u + tau d at other exponents
+// ----------------------------------------------------------------------------
+// A trial at q != 4 needs powers of |phi| that are no polynomials in tau, but
+// what they multiply is: p, G = P2|grad phi|^2, V = P2(W) (or, on the e_u
+// branch, the raw W, with E = P2(W / sqrt S)) are quadratic in tau, and
+// S = P2(|phi|^2) too.  The setup forms the coefficient fields once; a trial
+// reads them in the x stage that forms its products, and transforms only
+// those: 3 forward transforms at q = 6 and 3 forward, 1 inverse at q = 8 (8
+// forward, 3 inverse on the e_u branch) against 12 forward and 20 inverse
+// (11 and 18) of a whole R evaluation.  At 512^3 q = 6 mixed a trial takes
+// 4.2 ms instead of 18 (bound by the x stage's read of 23 fields, 0.79 of
+// the copy rate) and a CG iteration 138 instead of 383; two iterations at
+// 256^3 q = 6 FP64 take 83 instead of 187 ms with their transfers.
+
+// the fields of the setup and the trials fit next to what is allocated
+template <typename T>
+bool Engine<T>::lsg_fits() {
+    long need = 8;  // transform buffers and partials
+    for (int i = LU; i < LEND; ++i)
+        if ((i < LP + 3 || i >= LTS) && ((int)phys_.size() <= i || !phys_[i])) ++need;
+    if (need <= 8) return true;
+    size_t fr = 0, tot = 0;
+    MLQ_CUDA(cudaMemGetInfo(&fr, &tot));
+    return (double)need * (double)n3 * sizeof(T) < 0.8 * (double)fr;
+}
+
+template <typename T>
+void Engine<T>::lsg_setup(const SVec* u, const SVec* d, double tau0) {
+    ls_free_val_ = -1;
+    ls_dev_ = false;
+    ls_dev_alloc();
+    const LsFields lf = ls_fields(u, d);
+    if (use_e_u) {
+        std::vector<int> out;
+        for (int k = 0; k < 9; ++k) out.push_back(LW + k);
+        pointwise(FLSWRaw{}, lf.all, out);
+    } else {
+        ls_w_fields(lf);
+    }
+    ls_qg_fields(lf, true);
+    lsg_ud_ = lf.ud;
+    ls_interval_dev(tau0);
+}
+
+// ||phi||_q^q = <|phi|^{q/2}, |phi|^{q/2}>: the last product of the |phi|^k
+// chain is only summed (Parseval in the band that dealiases it), so it needs
+// no inverse transform.  Returns the result slot.
+template <typename T>
+int Engine<T>::lsg_power_sq(double k) {
+    FwdOut o;
+    o.red_self = 0;
+    constexpr int DST = 130;
+    if (k + MACH_EPSILON >= 2.0 && !memo_.count(k)) {
+        const double k2 = k - 2.0;
+        if (k2 != 0.0 && k2 + MACH_EPSILON < 2.0 && band_cut_for_order(n, k2) >= n / 2) {
+            FAPow f;
+            f.k = k2;
+            fwd(b2, f, {pa_, ps_}, {o}, DST);
+            return DST;
+        }
+        if (k2 != 0.0) {
+            PowField prev = chain(k2);
+            ensure_phys(prev);
+            fwd(b2, FMul{}, {pa_, prev.phys}, {o}, DST);
+            return DST;
+        }
+    } else if (!memo_.count(k)) {
+        const int c = band_cut_for_order(n, k);
+        if (c < n / 2) {
+            FGPow f;
+            f.k = k;
+            f.thresh = 0;
+            fwd(make_band(c), f, {ps_}, {o}, DST);
+            return DST;
+        }
+    }
+    PowField f = chain(k);
+    ensure_phys(f);
+    pointwise(FSqRed{}, {f.phys}, {}, 20);
+    return 20;
+}
+
+template <typename T>
+void Engine<T>::lsg_trial(double tau, double out[3], double* lqq) {
+    const double q = P.q, cv = P.visc_coef * P.visc, cp = P.press_coef;
+    chain_reset();
+    struct Sources {  // the chain reads this trial's S and A
+        int &s, &a;
+        Sources(int& s_, int& a_) : s(s_), a(a_) { s = LTS; a = LTA; }
+        ~Sources() { s = PS; a = PA; }
+    } src(ps_, pa_);
+    const std::vector<int> s3 = {ls_phys(0), ls_phys(1), ls_phys(2)};
+    const bool needA = q - 2.0 + MACH_EPSILON >= 2.0 || q / 2.0 + MACH_EPSILON >= 2.0;
+    const bool raw_a4 = q - 4.0 + MACH_EPSILON < 2.0;  // |phi|^{q-4} is outside the band (q branch)
+    if (needA && ls_clamp_free(tau)) {
+        // S(tau) >= 0 at every point: A = P2(max(S, 0)) = S
+        ++ls_poly_trials_;
+        FPolyS f;
+        f.tau = tau;
+        pointwise(f, s3, {LTS, LTA});
+        const long nsp = (long)b2.nb * b2.nb * b2.nx;
+        cudaEvent_t ev = prof_mark();
+        spec_poly3_kernel<cpx<T>><<<grid_for(nsp, 256), 256, 0, stream>>>(
+            wspec(WA), wspec(ls_wspec(0)), wspec(ls_wspec(1)), wspec(ls_wspec(2)), nsp, 1.0, tau, tau * tau, nullptr);
+        launched("spec_poly", 4.0 * nsp * sizeof(cpx<T>), ev);
+    } else {
+        ++ls_fft_trials_;
+        FPolyS1 f;
+        f.tau = tau;
+        pointwise(f, s3, {LTS});
+        if (needA) {
+            FwdOut oA;
+            oA.spec = wspec(WA);
+            oA.spec_f64 = wf64<T>();
+            oA.phys_out = LTA;
+            fwd(b2, FGSq{}, {LTS}, {oA});
+        }
+    }
+    std::vector<int> pud = {LP, LP + 1, LP + 2};
+    pud.insert(pud.end(), lsg_ud_.begin(), lsg_ud_.end());
+    FwdOut o[4];
+    const int ws[4] = {WT, WT + 1, WT + 2, WTA2};
+    for (int i = 0; i < 4; ++i) {
+        o[i].spec = wspec(ws[i]);
+        o[i].spec_f64 = wf64<T>();
+    }
+    std::vector<std::pair<const cpx<T>*, const cpx<T>*>> pr;
+    if (use_e_u) {
+        PowField a2 = chain(q - 2.0);
+        ensure_phys(a2);
+        FLSE fe;
+        fe.tau = tau;
+        FwdOut oE[3];
+        std::vector<int> in;
+        for (int k = 0; k < 9; ++k) in.push_back(LW + k);
+        in.push_back(LTS);
+        for (int j = 0; j < 3; ++j) oE[j].phys_out = LE + j;
+        fwd(b2, fe, in, {oE[0], oE[1], oE[2]});
+        in = {LE, LE + 1, LE + 2};
+        in.insert(in.end(), pud.begin(), pud.end());
+        for (int k : {(int)LTS, a2.phys, (int)LG, LG + 1, LG + 2}) in.push_back(k);
+        FLSTrialE f;
+        f.tau = tau;
+        fwd(b2, f, in, {o[0], o[1], o[2], o[3]}, -1, 16);
+        pr = {{wspec(WT + 1), wspec(WT + 2)}, {wspec(WT), wspec(WTA2)}};
+    } else {
+        PowField a4 = chain(q - 4.0);
+        ensure_phys(a4);
+        const bool direct = q - 2.0 + MACH_EPSILON < 2.0;
+        int a = LTA;
+        if (direct) {
+            PowField a2 = chain(q - 2.0);
+            ensure_phys(a2);
+            a = a2.phys;
+        }
+        std::vector<int> in;
+        for (int k = 0; k < 9; ++k) in.push_back(LV + k);
+        in.insert(in.end(), pud.begin(), pud.end());
+        for (int k : {a4.phys, a, (int)LG, LG + 1, LG + 2}) in.push_back(k);
+        pr = {{wspec(WT + 1), wspec(WT + 2)}};
+        if (raw_a4) {
+            FLSTrial<true> f;
+            f.tau = tau;
+            f.direct = direct;
+            fwd(b2, f, in, {o[1], o[2], o[0], o[3]}, -1, 16);
+            pr.push_back({wspec(WT), wspec(WTA2)});
+        } else {
+            FLSTrial<false> f;
+            f.tau = tau;
+            f.direct = direct;
+            fwd(b2, f, in, {o[1], o[2]}, -1, 16);
+        }
+    }
+    const int slot = lsg_power_sq(q / 2.0);
+    sdots(*this, pr, 0);
+    fetch_results();
+    const double I1 = h_results[16], I2 = use_e_u || raw_a4 ? h_results[1] : h_results[17], I3 = h_results[0];
+    const double R1 = -cv * I1;              // (1318)
+    const double R2 = -cv * (q - 2.0) * I2;  // (1333)
+    const double R3 = cp * (q - 2.0) * I3;   // (1352)
+    out[0] = R1 + R2 + R3;
+    out[1] = R1 + R2;
+    out[2] = R3;
+    if (lqq) *lqq = h_results[slot];
 }
 
 // ----------------------------------------------------------------------------

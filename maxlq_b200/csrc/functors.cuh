@@ -57,7 +57,11 @@ struct FGPow {
         const T s = in[0];
         const double g = s <= T(0) ? 0.0 : sqrt((double)s);
         double v;
-        if (thresh)
+        if (k == 1.0)  // the powers of q = 3 and 6 without pow, whose FP64
+            v = g;     // arithmetic bounds the kernel
+        else if (k == 1.5)
+            v = g * sqrt(g);
+        else if (thresh)
             v = fabs(g) < MACH_EPSILON ? 0.0 : pow(g, k);
         else
             v = pow(g, k);
@@ -527,6 +531,136 @@ struct FLSRed {
                 for (int b = 0; b < 3; ++b)
                     acc[6 + 3 * (2 * a + cc) + b] +=
                         p[a] * (c[cc][0] * V[b][0] + c[cc][1] * V[b][1] + c[cc][2] * V[b][2]);
+    }
+};
+
+// ---- trials at other exponents (q != 4, and the e_u branch) ------------------
+// S(tau) alone.  inputs s0, s1, s2
+struct FPolyS1 {
+    static constexpr int NIN = 3, NOUT = 1, NRED = 0;
+    double tau;
+    template <typename T>
+    __device__ void operator()(const T* in, T* out, double*) const {
+        const T t = (T)tau;
+        out[0] = in[0] + t * (in[1] + t * in[2]);
+    }
+};
+
+// A g^k, g = sqrt(max(S, 0)), for a power 0 < k <= 1 that no dealias follows
+// (calc_gk_order2 2309-2310 with 2300-2304).  inputs A, S
+struct FAPow {
+    static constexpr int NIN = 2, NOUT = 1, NRED = 0;
+    double k;
+    template <typename T>
+    __device__ void operator()(const T* in, T* out, double*) const {
+        const T s = in[1];
+        const T g = s <= T(0) ? T(0) : sqrt(s);
+        out[0] = in[0] * (k == 1.0 ? g : (T)pow((double)g, k));
+    }
+};
+
+// The tau^a coefficients of W_j = sum_i phi_i d_j phi_i before the dealias, at
+// 3a + j.  inputs u(3), Du(9), d(3), Dd(9)
+struct FLSWRaw {
+    static constexpr int NIN = 24, NOUT = 9, NRED = 0;
+    template <typename T>
+    __device__ void operator()(const T* in, T* out, double*) const {
+        const T* u = in;
+        const T* du = in + 3;
+        const T* d = in + 12;
+        const T* dd = in + 15;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            T w0 = 0, w1 = 0, w2 = 0;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                w0 += u[i] * du[3 * i + j];
+                w1 += u[i] * dd[3 * i + j] + d[i] * du[3 * i + j];
+                w2 += d[i] * dd[3 * i + j];
+            }
+            out[j] = w0;
+            out[3 + j] = w1;
+            out[6 + j] = w2;
+        }
+    }
+};
+
+// E_j = sum_i e_i d_j phi_i = W_j(tau) / sqrt|S|, 0 where the norm is below
+// MACH_EPSILON (unit_vec).  inputs W_aj at 3a + j (9), S(tau)
+struct FLSE {
+    static constexpr int NIN = 10, NOUT = 3, NRED = 0;
+    double tau;
+    template <typename T>
+    __device__ void operator()(const T* in, T* out, double*) const {
+        const T t = (T)tau;
+        const T nrm = sqrt(fabs(in[9]));
+        const bool zero = (double)nrm < MACH_EPSILON;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const T w = in[j] + t * (in[3 + j] + t * in[6 + j]);
+            out[j] = zero ? T(0) : w / nrm;
+        }
+    }
+};
+
+// q branch of a trial: out p a4 and phi . V (the two factors of R3), and the
+// R1 and R2 integrands, which need no transform of their own where they are
+// integrated against a field of the band, on which the dealias acts as the
+// identity: P2(A a4) against G, and P2(sum V^2) against a4.  a2 of the
+// reference is P2(A a4), or, with `direct`, the field given in A's place.
+// RAW: a4 is an undealiased power (0 < q - 4 < 2, or q < 4), so sum V^2 and a4
+// are outputs too.  inputs V_aj at 3a + j (9), p_a (3), u(3), d(3), a4, A, G_a (3)
+template <bool RAW>
+struct FLSTrial {
+    static constexpr int NIN = 23, NOUT = RAW ? 4 : 2, NRED = RAW ? 1 : 2;
+    double tau;
+    int direct;
+    template <typename T>
+    __device__ void operator()(const T* in, T* out, double* acc) const {
+        const T t = (T)tau;
+        T v2 = 0, uv = 0;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const T v = in[j] + t * (in[3 + j] + t * in[6 + j]);
+            v2 += v * v;
+            uv += (in[12 + j] + t * in[15 + j]) * v;
+        }
+        const T p = in[9] + t * (in[10] + t * in[11]);
+        const T g = in[20] + t * (in[21] + t * in[22]);
+        const T a4 = in[18], a = in[19];
+        out[0] = p * a4;
+        out[1] = uv;
+        acc[0] += (double)(direct ? a : a * a4) * (double)g;
+        if constexpr (RAW) {
+            out[2] = v2;
+            out[3] = a4;
+        } else {
+            acc[1] += (double)a4 * (double)v2;
+        }
+    }
+};
+
+// e_u branch of a trial: out sum E^2, p a2, e . E and a2, and the R1
+// integrand a2 G.  inputs E(3), p_a (3), u(3), d(3), S(tau), a2, G_a (3)
+struct FLSTrialE {
+    static constexpr int NIN = 17, NOUT = 4, NRED = 1;
+    double tau;
+    template <typename T>
+    __device__ void operator()(const T* in, T* out, double* acc) const {
+        const T t = (T)tau;
+        const T nrm = sqrt(fabs(in[12]));
+        T e2 = 0, ue = 0;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            e2 += in[j] * in[j];
+            ue += (in[6 + j] + t * in[9 + j]) * in[j];
+        }
+        const T a2 = in[13];
+        out[0] = e2;
+        out[1] = (in[3] + t * (in[4] + t * in[5])) * a2;
+        out[2] = (double)nrm < MACH_EPSILON ? T(0) : ue / nrm;
+        out[3] = a2;
+        acc[0] += (double)a2 * (double)(in[14] + t * (in[15] + t * in[16]));
     }
 };
 

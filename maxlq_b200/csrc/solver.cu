@@ -91,14 +91,18 @@ class Solver : public SolverBase {
     // Line-search trials go through the polynomial path when q = 4: setup
     // once per (base, dir), then one transform per trial.
     bool ls_ready = false;
+    bool lsg_ready = false;  // the same at q != 4
     // tau_near: a step the trials will visit the neighbourhood of (the
     // previous step in the CG loop), for the setup's clamp-free intervals
     void ls_begin(const SVec* base, const SVec* dir, double tau_near = 0.0) {
         trials.clear();
-        ls_ready = false;
+        ls_ready = lsg_ready = false;
         if (e.ls_ok() && dir && e.ls_fits()) {
             e.ls_setup(base, dir, tau_near);
             ls_ready = true;
+        } else if (e.lsg_ok() && dir && e.lsg_fits()) {
+            e.lsg_setup(base, dir, tau_near);
+            lsg_ready = true;
         }
     }
     Trial trial(const SVec* base, const SVec* dir, double tau) {
@@ -107,6 +111,8 @@ class Solver : public SolverBase {
         Trial t;
         if (ls_ready)
             e.ls_trial(tau, t.R, &t.lqq);
+        else if (lsg_ready)
+            e.lsg_trial(tau, t.R, &t.lqq);
         else
             e.R_eval(base, dir, tau, t.R, &t.lqq);
         trials[tau] = t;
@@ -303,7 +309,7 @@ class Solver : public SolverBase {
         // vector transport of gu1 and d1 to the new point (324-328)
         double ir[2];
         const SVec* xi[2] = {g1, d1};
-        ls_ready = false;
+        ls_ready = lsg_ready = false;
         double lqw;
         if (e.P.use_riemannian_geometry)
             lqw = e.transport_pieces(u, d1, tau1, xi, 2, ir);
