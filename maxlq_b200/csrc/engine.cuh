@@ -436,9 +436,16 @@ class Engine : public EngineBase {
     // are not.  Resident mode only; MLQ_REUSE=0 evaluates R whole per trial.
     bool lsg_ok() const { return !ls_ok() && !slab_ && reuse_on_; }
     bool lsg_fits();
+    bool lsg_fit_ = false;
     void lsg_setup(const SVec* u, const SVec* d, double tau0 = 0.0);
     void lsg_trial(double tau, double out[3], double* lqq);
     int lsg_power_sq(double k);
+    // even q (6 and 8): the coefficients of the trial's integrals where S(tau)
+    // >= 0 at every point (at q = 6 the norm takes one transform per trial)
+    bool lsg_poly_ok() const { return !use_e_u && (P.q == 6.0 || P.q == 8.0); }
+    void lsg_poly_setup();
+    bool lsg_poly_fetched_ = false;
+    double lsg_i1_[9], lsg_i2_[9], lsg_i3_[10], lsg_nrm_[9];
     std::vector<int> lsg_ud_;  // physical fields of u and d in this line search
     // parts of the setups
     struct LsFields {

@@ -1376,6 +1376,7 @@ template <typename T>
 void Engine<T>::release_io_buffers() {
     pu_of_ = nullptr;
     pm_ = PhysMemo{};
+    lsg_fit_ = false;
     for (auto* v : {&phys_}) {
         for (auto*& p : *v) {
             if (p) free_dev(p);
@@ -1468,8 +1469,15 @@ enum : int {
     LG = 112,   // 112..114
     LW = 115,   // 115..123
     LE = 124,   // 124..126
-    LEND = 127,
+    LC = 127,   // 127..131 coefficients of |phi|^{q-4} at q = 8
+    LEND = 132,
     WTA2 = 54,  // work spectrum of |phi|^{q-2} (e_u branch)
+    WLC = 55,   // 55..59 spectra of C
+    WLP = 60,   // 60..66 coefficients of P2(p C)
+    WLU = 67,   // 67..70 coefficients of P2(phi . V)
+    RPOLY = 160,  // result slots: 18 of FLSPolyRed, 10 of I3, 9 of the norm
+    RI3 = 180,
+    RNRM = 190,
 };
 }  // namespace
 
@@ -2900,16 +2908,25 @@ void Engine<T>::ls_trial(double tau, double out[3], double* lqq) {
 // the copy rate) and a CG iteration 138 instead of 383; two iterations at
 // 256^3 q = 6 FP64 take 83 instead of 187 ms with their transfers.
 
-// the fields of the setup and the trials fit next to what is allocated
+// The fields of the setup and the trials fit next to what is allocated.
+// Asked until they do, since cudaMemGetInfo stalls for up to 100 ms at times;
+// the first search allocates them.
 template <typename T>
 bool Engine<T>::lsg_fits() {
+    if (lsg_fit_) return true;
     long need = 8;  // transform buffers and partials
-    for (int i = LU; i < LEND; ++i)
-        if ((i < LP + 3 || i >= LTS) && ((int)phys_.size() <= i || !phys_[i])) ++need;
-    if (need <= 8) return true;
+    for (int i = LU; i < LEND; ++i) {
+        const bool used = i < LP + 3 ? (!use_e_u || i < LV || i >= LP)
+                          : i < LTS  ? false
+                          : i < LW   ? true
+                          : i < LC   ? use_e_u
+                                     : lsg_poly_ok() && P.q == 8.0;
+        if (used && ((int)phys_.size() <= i || !phys_[i])) ++need;
+    }
     size_t fr = 0, tot = 0;
     MLQ_CUDA(cudaMemGetInfo(&fr, &tot));
-    return (double)need * (double)n3 * sizeof(T) < 0.8 * (double)fr;
+    lsg_fit_ = (double)need * (double)n3 * sizeof(T) < 0.8 * (double)fr;
+    return lsg_fit_;
 }
 
 template <typename T>
@@ -2927,7 +2944,106 @@ void Engine<T>::lsg_setup(const SVec* u, const SVec* d, double tau0) {
     }
     ls_qg_fields(lf, true);
     lsg_ud_ = lf.ud;
+    if (lsg_poly_ok()) lsg_poly_setup();
     ls_interval_dev(tau0);
+}
+
+// The Parseval products of two polynomial spectra, by power of tau: one pass
+// over the NA + NB spectra (a == b: one array of NA) instead of NA NB scalar
+// products of pairs.
+template <typename T, int NA, int NB>
+struct PolyDotArgs {
+    SpecGeom g;
+    const cpx<T>* a[NA];
+    const cpx<T>* b[NB];
+    double* partials;
+};
+template <typename T, int NA, int NB, bool SAME>
+__global__ void __launch_bounds__(RED_THREADS) spec_polydot_kernel(PolyDotArgs<T, NA, NB> a) {
+    constexpr int NR = NA + NB - 1;
+    double acc[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) acc[r] = 0.0;
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.g.ncomp; i += (long)gridDim.x * blockDim.x) {
+        const double w = kx_weight(a.g.n, (int)(i % a.g.nx));
+        cpx<T> x[NA], y[NB];
+#pragma unroll
+        for (int k = 0; k < NA; ++k) x[k] = a.a[k][i];
+#pragma unroll
+        for (int k = 0; k < NB; ++k) y[k] = SAME ? x[k] : a.b[k][i];
+#pragma unroll
+        for (int k = 0; k < NA; ++k)
+#pragma unroll
+            for (int m = 0; m < NB; ++m)
+                acc[k + m] += w * ((double)x[k].x * (double)y[m].x + (double)x[k].y * (double)y[m].y);
+    }
+    block_reduce_store<NR>(acc, a.partials, blockIdx.x);
+}
+template <typename T, int NA, int NB, bool SAME>
+static void polydot(Engine<T>& e, int wa, int wb, int dst) {
+    PolyDotArgs<T, NA, NB> a;
+    a.g = e.geom(e.b2);
+    for (int k = 0; k < NA; ++k) a.a[k] = e.wspec(wa + k);
+    for (int k = 0; k < NB; ++k) a.b[k] = e.wspec(wb + k);
+    const int grid = grid_for(a.g.ncomp, RED_THREADS, 148 * 4);
+    e.ensure_partials((long)grid * (NA + NB - 1));
+    a.partials = e.d_partials;
+    cudaEvent_t ev = e.prof_mark();
+    spec_polydot_kernel<T, NA, NB, SAME><<<grid, RED_THREADS, 0, e.stream>>>(a);
+    e.launched("spec_sdot", (double)(SAME ? NA : NA + NB) * a.g.ncomp * sizeof(cpx<T>), ev);
+    e.finalize(grid, NA + NB - 1, 1.0, dst);
+}
+
+// Even q: I1 = int A C G, I2 = int C sum V^2, I3 = <P2(p C), P2(phi . V)> and,
+// at q = 8, ||phi||^8 = <C, C> as polynomials in tau (C = |phi|^{q-4}).  The
+// setup pays 9 forward transforms at q = 6, 16 forward and 5 inverse at q = 8;
+// each clamp-free trial then saves its 3 (q = 6: 2) forward transforms and its
+// pass over 23 fields.  A 512^3 q = 6 mixed iteration takes 64 instead of 138
+// ms (a trial 1.1 instead of 4.2), three iterations at 48^3 q = 8 FP64 4.5
+// instead of 9.7 with their transfers.  Outside the clamp-free intervals the
+// trials above remain.
+template <typename T>
+void Engine<T>::lsg_poly_setup() {
+    lsg_poly_fetched_ = false;
+    const bool q8 = P.q == 8.0;
+    const int s3[3] = {ls_phys(0), ls_phys(1), ls_phys(2)};
+    auto spec_out = [&](int w) {
+        FwdOut o;
+        o.spec = wspec(w);
+        o.spec_f64 = wf64<T>();
+        return o;
+    };
+    std::vector<int> red, pc = {LP, LP + 1, LP + 2};
+    for (int k = 0; k < 9; ++k) red.push_back(LV + k);
+    for (int a = 0; a < 3; ++a) red.push_back(LG + a);
+    if (q8) {
+        std::vector<FwdOut> o;
+        for (int k = 0; k < 5; ++k) {
+            o.push_back(spec_out(WLC + k));
+            o[k].phys_out = LC + k;
+            red.push_back(LC + k);
+            pc.push_back(LC + k);
+        }
+        fwd(b2, FLSC2{}, {s3[0], s3[1], s3[2]}, o);
+        polydot<T, 5, 5, true>(*this, WLC, WLC, RNRM);
+    }
+    for (int a = 0; a < 3; ++a) {
+        red.push_back(s3[a]);
+        if (!q8) pc.push_back(s3[a]);
+    }
+    std::vector<int> uv = lsg_ud_;
+    for (int k = 0; k < 9; ++k) uv.push_back(LV + k);
+    fwd(b2, FLSUV{}, uv, {spec_out(WLU), spec_out(WLU + 1), spec_out(WLU + 2), spec_out(WLU + 3)});
+    if (q8) {
+        pointwise(FLSPolyRed<5>{}, red, {}, RPOLY);
+        fwd(b2, FLSPC8A{}, pc, {spec_out(WLP), spec_out(WLP + 1), spec_out(WLP + 2), spec_out(WLP + 3)});
+        fwd(b2, FLSPC8B{}, pc, {spec_out(WLP + 4), spec_out(WLP + 5), spec_out(WLP + 6)});
+        polydot<T, 7, 4, false>(*this, WLP, WLU, RI3);
+    } else {
+        pointwise(FLSPolyRed<3>{}, red, {}, RPOLY);
+        fwd(b2, FLSPC6{}, pc, {spec_out(WLP), spec_out(WLP + 1), spec_out(WLP + 2), spec_out(WLP + 3), spec_out(WLP + 4)});
+        polydot<T, 5, 4, false>(*this, WLP, WLU, RI3);
+    }
 }
 
 // ||phi||_q^q = <|phi|^{q/2}, |phi|^{q/2}>: the last product of the |phi|^k
@@ -2980,7 +3096,43 @@ void Engine<T>::lsg_trial(double tau, double out[3], double* lqq) {
     const std::vector<int> s3 = {ls_phys(0), ls_phys(1), ls_phys(2)};
     const bool needA = q - 2.0 + MACH_EPSILON >= 2.0 || q / 2.0 + MACH_EPSILON >= 2.0;
     const bool raw_a4 = q - 4.0 + MACH_EPSILON < 2.0;  // |phi|^{q-4} is outside the band (q branch)
-    if (needA && ls_clamp_free(tau)) {
+    const bool free_tau = needA && ls_clamp_free(tau);
+    auto result = [&](double I1, double I2, double I3) {
+        const double R1 = -cv * I1;              // (1318)
+        const double R2 = -cv * (q - 2.0) * I2;  // (1333)
+        const double R3 = cp * (q - 2.0) * I3;   // (1352)
+        out[0] = R1 + R2 + R3;
+        out[1] = R1 + R2;
+        out[2] = R3;
+    };
+    if (free_tau && lsg_poly_ok()) {
+        ++ls_poly_trials_;
+        const int nc = q == 8.0 ? 5 : 3;
+        if (nc == 3) {
+            FLSS32 f;
+            f.tau = tau;
+            FwdOut o;
+            o.red_self = 0;
+            fwd(b2, f, s3, {o}, 130);
+        }
+        if (nc == 3 || !lsg_poly_fetched_) fetch_results();
+        if (!lsg_poly_fetched_) {
+            std::copy(h_results + RPOLY, h_results + RPOLY + nc + 4, lsg_i1_);
+            std::copy(h_results + RPOLY + nc + 4, h_results + RPOLY + 2 * (nc + 4), lsg_i2_);
+            std::copy(h_results + RI3, h_results + RI3 + nc + 5, lsg_i3_);
+            std::copy(h_results + RNRM, h_results + RNRM + 9, lsg_nrm_);
+            lsg_poly_fetched_ = true;
+        }
+        auto poly = [&](const double* c, int m) {
+            double v = 0.0;
+            for (int k = m - 1; k >= 0; --k) v = v * tau + c[k];
+            return v;
+        };
+        result(poly(lsg_i1_, nc + 4), poly(lsg_i2_, nc + 4), poly(lsg_i3_, nc + 5));
+        if (lqq) *lqq = nc == 3 ? h_results[130] : poly(lsg_nrm_, 9);
+        return;
+    }
+    if (free_tau) {
         // S(tau) >= 0 at every point: A = P2(max(S, 0)) = S
         ++ls_poly_trials_;
         FPolyS f;
@@ -3062,13 +3214,7 @@ void Engine<T>::lsg_trial(double tau, double out[3], double* lqq) {
     const int slot = lsg_power_sq(q / 2.0);
     sdots(*this, pr, 0);
     fetch_results();
-    const double I1 = h_results[16], I2 = use_e_u || raw_a4 ? h_results[1] : h_results[17], I3 = h_results[0];
-    const double R1 = -cv * I1;              // (1318)
-    const double R2 = -cv * (q - 2.0) * I2;  // (1333)
-    const double R3 = cp * (q - 2.0) * I3;   // (1352)
-    out[0] = R1 + R2 + R3;
-    out[1] = R1 + R2;
-    out[2] = R3;
+    result(h_results[16], use_e_u || raw_a4 ? h_results[1] : h_results[17], h_results[0]);
     if (lqq) *lqq = h_results[slot];
 }
 

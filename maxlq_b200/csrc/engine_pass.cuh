@@ -13,7 +13,8 @@
     X(P, T, N, FG3<false>) X(P, T, N, FG3<true>) X(P, T, N, FC3) X(P, T, N, FLSS) X(P, T, N, FLSS12)              \
     X(P, T, N, FLSW<0>) X(P, T, N, FLSW<1>) X(P, T, N, FLSQG) X(P, T, N, FLSA) X(P, T, N, FAPow)           \
     X(P, T, N, FLSE) X(P, T, N, FLSTrial<false>) X(P, T, N, FLSTrial<true>)                               \
-    X(P, T, N, FLSTrialE)
+    X(P, T, N, FLSTrialE) X(P, T, N, FLSC2) X(P, T, N, FLSPC6) X(P, T, N, FLSPC8A) X(P, T, N, FLSPC8B)            \
+    X(P, T, N, FLSUV) X(P, T, N, FLSS32)
 #define MLQ_PASS_X(P, T, N, F) P template void Engine<T>::xfwd_c<N, F>(XFwdArgs<T>&, const F&);
 
 // P: `extern` (declaration) or nothing (definition)

@@ -640,6 +640,109 @@ struct FLSTrial {
     }
 };
 
+// ---- even q >= 6: the whole trial polynomial in tau ---------------------------
+// Where S(tau) >= 0 at every point, A = S(tau) and |phi|^{q-4} = C(tau) is a
+// polynomial field too: C = A at q = 6 (NC = 3 coefficient fields), C = P2(A A)
+// at q = 8 (NC = 5).
+
+// The coefficients of P2(A A) before the dealias.  inputs S_a (3)
+struct FLSC2 {
+    static constexpr int NIN = 3, NOUT = 5, NRED = 0;
+    template <typename T>
+    __device__ void operator()(const T* in, T* out, double*) const {
+        out[0] = in[0] * in[0];
+        out[1] = T(2) * (in[0] * in[1]);
+        out[2] = in[1] * in[1] + T(2) * (in[0] * in[2]);
+        out[3] = T(2) * (in[1] * in[2]);
+        out[4] = in[2] * in[2];
+    }
+};
+
+// Coefficients K0 .. K0 + KN - 1 of p C.  inputs p_a (3), C (NC)
+template <int NC, int K0, int KN>
+struct FLSPC {
+    static constexpr int NIN = 3 + NC, NOUT = KN, NRED = 0;
+    template <typename T>
+    __device__ void operator()(const T* in, T* out, double*) const {
+#pragma unroll
+        for (int k = 0; k < KN; ++k) {
+            T v = 0;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const int b = K0 + k - a;
+                if (b >= 0 && b < NC) v += in[a] * in[3 + b];
+            }
+            out[k] = v;
+        }
+    }
+};
+
+using FLSPC6 = FLSPC<3, 0, 5>;
+using FLSPC8A = FLSPC<5, 0, 4>;  // in two launches: seven parked FP64 outputs
+using FLSPC8B = FLSPC<5, 4, 3>;  // exceed a block's shared memory
+
+// Coefficients of phi . V.  inputs u(3), d(3), V_aj at 3a + j (9)
+struct FLSUV {
+    static constexpr int NIN = 15, NOUT = 4, NRED = 0;
+    template <typename T>
+    __device__ void operator()(const T* in, T* out, double*) const {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            T v = 0;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                if (m < 3) v += in[j] * in[6 + 3 * m + j];
+                if (m > 0) v += in[3 + j] * in[6 + 3 * (m - 1) + j];
+            }
+            out[m] = v;
+        }
+    }
+};
+
+// Coefficients of the R1 and R2 integrands A C G (slots 0 .. NC+3) and
+// C sum_j V_j^2 (NC+4 ..).  inputs V_aj (9), G_a (3), C (NC) and, for NC = 5,
+// S_a (3) (C = A for NC = 3)
+template <int NC>
+struct FLSPolyRed {
+    static constexpr int NIN = NC == 3 ? 15 : 20, NOUT = 0, NRED = 2 * (NC + 4);
+    template <typename T>
+    __device__ void operator()(const T* in, T*, double* acc) const {
+        const T* S = NC == 3 ? in + 12 : in + 12 + NC;
+        double s[3], c[NC], v2[5] = {0, 0, 0, 0, 0}, sg[5] = {0, 0, 0, 0, 0};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) s[a] = (double)S[a];
+#pragma unroll
+        for (int b = 0; b < NC; ++b) c[b] = (double)in[12 + b];
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                sg[a + b] += s[a] * (double)in[9 + b];
+#pragma unroll
+                for (int j = 0; j < 3; ++j) v2[a + b] += (double)in[3 * a + j] * (double)in[3 * b + j];
+            }
+#pragma unroll
+        for (int b = 0; b < NC; ++b)
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                acc[b + k] += c[b] * sg[k];
+                acc[NC + 4 + b + k] += c[b] * v2[k];
+            }
+    }
+};
+
+// S^{3/2}: the norm's A g at q = 6 where A = S.  inputs S_a (3)
+struct FLSS32 {
+    static constexpr int NIN = 3, NOUT = 1, NRED = 0;
+    double tau;
+    template <typename T>
+    __device__ void operator()(const T* in, T* out, double*) const {
+        const T t = (T)tau;
+        const T s = in[0] + t * (in[1] + t * in[2]);
+        out[0] = s <= T(0) ? T(0) : s * sqrt(s);
+    }
+};
+
 // e_u branch of a trial: out sum E^2, p a2, e . E and a2, and the R1
 // integrand a2 G.  inputs E(3), p_a (3), u(3), d(3), S(tau), a2, G_a (3)
 struct FLSTrialE {
