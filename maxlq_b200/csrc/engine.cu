@@ -131,7 +131,7 @@ void EngineBase::ensure_partials(long cnt) {
 
 void EngineBase::finalize(int nblocks, int nr, double scale, int dst, bool accumulate) {
     cudaEvent_t ev = prof_mark();
-    finalize_partials_kernel<<<1, RED_THREADS, 0, stream>>>(d_partials, nblocks, nr, scale, d_results, dst,
+    finalize_partials_kernel<<<1, FIN_THREADS, 0, stream>>>(d_partials, nblocks, nr, scale, d_results, dst,
                                                            accumulate ? 1 : 0);
     launched("finalize", 8.0 * nblocks * nr, ev);
 }

@@ -1162,11 +1162,15 @@ void Engine<T>::pointwise(const F& f, const std::vector<int>& in, const std::vec
         a.out[o] = phys(out[o]);
         phys_written(out[o]);
     }
-    const int grid = grid_for(n3, RED_THREADS, 148 * 8);
+    // a reduction ends with a reduction over each block: no more blocks than
+    // are resident at once (FLSRed at 64^3: 25 us in 1024 blocks)
+    auto kern = pointwise_kernel<T, F>;
+    const int cap = F::NRED > 0 ? persistent_blocks((const void*)kern, RED_THREADS, 0) : 148 * 8;
+    const int grid = grid_for((n3 + 1) / 2, RED_THREADS, cap);
     ensure_partials((long)grid * std::max(F::NRED, 1));
     a.partials = d_partials;
     cudaEvent_t ev = prof_mark();
-    pointwise_kernel<T, F><<<grid, RED_THREADS, 0, stream>>>(a, f);
+    kern<<<grid, RED_THREADS, 0, stream>>>(a, f);
     launched("pointwise", (double)n3 * sizeof(T) * (F::NIN + F::NOUT), ev);
     if (F::NRED > 0 && fred_dst >= 0) finalize(grid, F::NRED, 1.0 / (double)n3, fred_dst);
 }
@@ -2577,6 +2581,42 @@ void Engine<T>::ls_interval_dev(double tau0) {
     ls_host_poly_ = false;
 }
 
+// The Parseval products of the S_i spectra with the G_a and with each other,
+// in one pass over the six (three passes of up to six pairs read 30: with the
+// two norms of an iteration 0.93 ms at 512^3 mixed, now 0.48).
+template <typename T>
+struct LsDotArgs {
+    SpecGeom g;
+    const cpx<T>* s[3];
+    const cpx<T>* x[3];
+    double* partials;
+};
+template <typename T>
+__global__ void __launch_bounds__(RED_THREADS) spec_ls_dot_kernel(LsDotArgs<T> a) {
+    double acc[15];
+#pragma unroll
+    for (int r = 0; r < 15; ++r) acc[r] = 0.0;
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.g.ncomp; i += (long)gridDim.x * blockDim.x) {
+        const double w = kx_weight(a.g.n, (int)(i % a.g.nx));
+        cpx<T> s[3], x[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            s[k] = a.s[k][i];
+            x[k] = a.x[k][i];
+        }
+        auto dot = [&](cpx<T> u, cpx<T> v) { return w * ((double)u.x * (double)v.x + (double)u.y * (double)v.y); };
+        int r = 9;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+#pragma unroll
+            for (int m = 0; m < 3; ++m) acc[3 * k + m] += dot(s[k], x[m]);
+#pragma unroll
+            for (int m = k; m < 3; ++m) acc[r++] += dot(s[k], s[m]);
+        }
+    }
+    block_reduce_store<15>(acc, a.partials, blockIdx.x);
+}
+
 template <typename T>
 void Engine<T>::ls_setup(const SVec* u, const SVec* d, double tau0) {
     ls_free_val_ = -1;
@@ -2597,17 +2637,22 @@ void Engine<T>::ls_setup(const SVec* u, const SVec* d, double tau0) {
         release_slots(LU, LS);
         release_slots(LV, LP + 3);
     }
-    // Parseval products for the transform-free trials
+    // Parseval products for the transform-free trials: <S_i, G_a> in slots
+    // 140..148, <S_i, S_j> in 149..154
     {
-        std::vector<std::pair<const cpx<T>*, const cpx<T>*>> p1, p2, p3;
-        for (int i = 0; i < 3; ++i)
-            for (int a = 0; a < 3; ++a) (i < 2 ? p1 : p2).push_back({wspec(ls_wspec(i)), wspec(WLG + a)});
-        for (int i = 0; i < 3; ++i)
-            for (int j = i; j < 3; ++j)
-                (p2.size() < 6 ? p2 : p3).push_back({wspec(ls_wspec(i)), wspec(ls_wspec(j))});
-        sdots(*this, p1, 140);
-        sdots(*this, p2, 146);
-        sdots(*this, p3, 152);
+        LsDotArgs<T> a;
+        a.g = geom(b2);
+        for (int i = 0; i < 3; ++i) {
+            a.s[i] = wspec(ls_wspec(i));
+            a.x[i] = wspec(WLG + i);
+        }
+        const int grid = grid_for(a.g.ncomp, RED_THREADS, 148 * 4);
+        ensure_partials((long)grid * 15);
+        a.partials = d_partials;
+        cudaEvent_t ev = prof_mark();
+        spec_ls_dot_kernel<T><<<grid, RED_THREADS, 0, stream>>>(a);
+        launched("spec_sdot", 6.0 * a.g.ncomp * sizeof(cpx<T>), ev);
+        finalize(grid, 15, 1.0, 140);
     }
     // the interval of tau around 0 on which S(tau) >= 0 everywhere
     if (ls_dev_) {  // on the device, with the coefficients: no host round trip
@@ -2647,7 +2692,6 @@ void Engine<T>::ls_setup(const SVec* u, const SVec* d, double tau0) {
         }
     }
     fetch_results();
-    // <S_i, G_a> in slots 140..148 (146.. holds i = 2), <S_i, S_j> in 149..154
     ls_assemble(h_results + 100, h_results + 140, h_results + 149, lo[0], hi[0], lo + 1, hi + 1, an.a, ls_c_);
     ls_host_poly_ = true;
 }

@@ -388,7 +388,7 @@ struct LsDevState {
     int ntr;
     int need;  // 0 none, 1 check of ptau pending, 2 transform of ptau pending
     double ptau;
-    double mtau[LS_MEMO], mR[LS_MEMO][3], mlqq[LS_MEMO];
+    double mtau[LS_MEMO], mR[LS_MEMO][3], mlqq[LS_MEMO], mJ[LS_MEMO];
     int mfft[LS_MEMO];
 };
 

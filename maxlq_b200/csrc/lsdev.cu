@@ -16,41 +16,54 @@ __device__ bool ls_memo_add(LsDevState* s, double tau, const double R[3], double
     s->mtau[k] = tau;
     for (int i = 0; i < 3; ++i) s->mR[k][i] = R[i];
     s->mlqq[k] = lqq;
+    s->mJ[k] = ls_J(R[1], R[2], lqq, s->par.q, s->par.B);
     s->mfft[k] = fft;
     s->ntr = k + 1;
     return true;
 }
 
+// What the controller reads, in shared memory: it is one thread, and a trial
+// is a chain of dependent reads of these.
+struct LsShared {
+    LsPoly poly;
+    LsParams par;
+    double tau[LS_MEMO], J[LS_MEMO];
+};
+
 // J(tau) from the table, or from the polynomials inside [tlo, thi];
 // anything else suspends the search at tau.
 struct DevEval {
     LsDevState* s;
+    LsShared* sh;
+    int n;  // entries of the table
     int count = 0;
     int err = 0;
     double ptau = 0.0;
     __device__ bool operator()(double tau, double* J) {
         ++count;
-        const LsParams& p = s->par;
+        const LsParams& p = sh->par;
         int k = -1;
-        for (int i = 0; i < s->ntr; ++i)
-            if (s->mtau[i] == tau) {
+        for (int i = 0; i < n; ++i)
+            if (sh->tau[i] == tau) {
                 k = i;
                 break;
             }
         if (k < 0) {
-            if (p.transform_trials || !ls_free(s->poly, tau)) {
+            if (p.transform_trials || !ls_free(sh->poly, tau)) {
                 ptau = tau;
                 return false;
             }
             double R[3], lqq;
-            ls_poly_R(s->poly, p.q, p.cv, p.cp, tau, R, &lqq);
+            ls_poly_R(sh->poly, p.q, p.cv, p.cp, tau, R, &lqq);
             if (!ls_memo_add(s, tau, R, lqq, 0)) {
                 err = LS_ERR_CAP;
                 return false;
             }
-            k = s->ntr - 1;
+            k = n++;
+            sh->tau[k] = tau;
+            sh->J[k] = s->mJ[k];
         }
-        *J = ls_J(s->mR[k][1], s->mR[k][2], s->mlqq[k], p.q, p.B);
+        *J = sh->J[k];
         if (isnan(*J)) {
             err = MLQ_ERR_NAN;
             return false;
@@ -68,32 +81,50 @@ __device__ void ls_stop(LsDevState* s, int status, cudaGraphConditionalHandle h_
 
 }  // namespace
 
+constexpr int LS_COEF_THREADS = 512;
+
 // The coefficients of this line search from the setup's sums (results[100..],
 // [140..], [149..]) and the per-block interval ends (partials, 2 per block);
 // clears the table for a new search.
-__global__ void ls_coef_kernel(LsDevState* s, const double* __restrict__ results,
-                               const double* __restrict__ partials, int nblocks, LsAnchorSet an) {
-    if (blockIdx.x != 0 || threadIdx.x >= 32) return;
-    // one warp: each lane takes every 32nd block, then a shuffle tree (max and
-    // min are exact, so any order gives the same ends)
-    constexpr int K = LS_ANCHORS + 1, W = 2 * K;
-    const int lane = threadIdx.x;
+__global__ void __launch_bounds__(LS_COEF_THREADS)
+    ls_coef_kernel(LsDevState* s, const double* __restrict__ results, const double* __restrict__ partials, int nblocks,
+                   LsAnchorSet an) {
+    // max and min are exact, so any order gives the same ends; one warp alone
+    // took 20 us over the 592 blocks of 64^3
+    constexpr int K = LS_ANCHORS + 1, W = 2 * K, NW = LS_COEF_THREADS / 32;
+    __shared__ double slo[NW][K], shi[NW][K];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double lo[K], hi[K];
+#pragma unroll
     for (int k = 0; k < K; ++k) {
         lo[k] = -1e300;
         hi[k] = 1e300;
     }
-    for (int g = lane; g < nblocks; g += 32)
+    for (int g = threadIdx.x; g < nblocks; g += LS_COEF_THREADS)
+#pragma unroll
         for (int k = 0; k < K; ++k) {
             lo[k] = fmax(lo[k], partials[W * g + 2 * k]);
             hi[k] = fmin(hi[k], partials[W * g + 2 * k + 1]);
         }
-    for (int k = 0; k < K; ++k)
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
         for (int o = 16; o > 0; o >>= 1) {
             lo[k] = fmax(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
             hi[k] = fmin(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
         }
-    if (lane != 0) return;
+        if (lane == 0) {
+            slo[warp][k] = lo[k];
+            shi[warp][k] = hi[k];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        for (int w = 1; w < NW; ++w) {
+            lo[k] = fmax(lo[k], slo[w][k]);
+            hi[k] = fmin(hi[k], shi[w][k]);
+        }
     ls_assemble(results + 100, results + 140, results + 149, lo[0], hi[0], lo + 1, hi + 1, an.a, s->poly);
     s->ntr = 0;
     s->need = 0;
@@ -106,6 +137,16 @@ __global__ void ls_coef_kernel(LsDevState* s, const double* __restrict__ results
 // table; ends the loop when the search completes (or fails), else leaves
 // the first tau without a value in ptau and opens the check branch.
 __global__ void ls_ctrl_kernel(LsDevState* s, cudaGraphConditionalHandle h_loop, cudaGraphConditionalHandle h_chk) {
+    __shared__ LsShared sh;
+    const int n = s->ntr;
+    for (int i = threadIdx.x; i < (int)(sizeof(LsPoly) / sizeof(double)); i += blockDim.x)
+        reinterpret_cast<double*>(&sh.poly)[i] = reinterpret_cast<const double*>(&s->poly)[i];
+    if (threadIdx.x == 0) sh.par = s->par;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        sh.tau[i] = s->mtau[i];
+        sh.J[i] = s->mJ[i];
+    }
+    __syncwarp();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     LsOut& o = s->out;
     if (o.status != LS_RUNNING) {
@@ -117,7 +158,7 @@ __global__ void ls_ctrl_kernel(LsDevState* s, cudaGraphConditionalHandle h_loop,
         return;
     }
     ++o.loops;
-    DevEval ev{s};
+    DevEval ev{s, &sh, n};
     double tb[2] = {0.0, 0.0}, x = 0.0, fx = 0.0;
     int mflag = 0;
     int r = ls_mnbrak(ev, s->par.tA0, s->par.tB0, tb, &mflag);
@@ -163,9 +204,10 @@ __global__ void ls_ctrl_kernel(LsDevState* s, cudaGraphConditionalHandle h_loop,
 // transform branch.
 __global__ void ls_check_kernel(LsDevState* s, const double* __restrict__ partials, int nblocks,
                                 cudaGraphConditionalHandle h_fft) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
     double mn = 1e300;
-    for (int g = 0; g < nblocks; ++g) mn = fmin(mn, partials[g]);
+    for (int g = threadIdx.x; g < nblocks; g += 32) mn = fmin(mn, partials[g]);
+    for (int o = 16; o > 0; o >>= 1) mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    if (threadIdx.x != 0 || blockIdx.x != 0) return;
     if (mn >= 0.0 && !s->par.transform_trials) {
         double R[3], lqq;
         ls_poly_R(s->poly, s->par.q, s->par.cv, s->par.cp, s->ptau, R, &lqq);
@@ -189,7 +231,7 @@ __global__ void ls_fft_kernel(LsDevState* s, const double* __restrict__ r) {
 
 void ls_launch_coef(LsDevState* s, const double* results, const double* partials, int nblocks, const LsAnchorSet& an,
                     cudaStream_t st) {
-    ls_coef_kernel<<<1, 32, 0, st>>>(s, results, partials, nblocks, an);
+    ls_coef_kernel<<<1, LS_COEF_THREADS, 0, st>>>(s, results, partials, nblocks, an);
 }
 void ls_launch_ctrl(LsDevState* s, cudaGraphConditionalHandle h_loop, cudaGraphConditionalHandle h_chk,
                     cudaStream_t st) {
