@@ -53,6 +53,7 @@ EngineBase::EngineBase(const mlq_params& p) : P(p) {
     MLQ_CUDA(cudaMemcpyAsync(d_tw, pool.data(), pool.size() * sizeof(cpx<double>), cudaMemcpyHostToDevice, stream));
     MLQ_CUDA(cudaStreamSynchronize(stream));
     d_results = (double*)dev_alloc(NRES * sizeof(double));
+    MLQ_CUDA(cudaMallocHost((void**)&h_results, NRES * sizeof(double)));
     MLQ_CUDA(cudaMemsetAsync(d_results, 0, NRES * sizeof(double), stream));
     MLQ_CUDA(cudaStreamSynchronize(stream));
     ensure_partials(1 << 20);
@@ -65,6 +66,7 @@ EngineBase::~EngineBase() {
     for (auto& kv : graphs_)
         if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
     for (auto& a : allocs_) cudaFree(a.first);
+    if (h_results) cudaFreeHost(h_results);
     if (stream) cudaStreamDestroy(stream);
 }
 
@@ -269,34 +271,34 @@ void EngineBase::retract(SVec* u, double cs, double tau, const SVec* d) {
         pm_.u = nullptr;  // the fields describe the old u, no longer stored
         pm_.ls = false;
         pm_.next = u;
+        pm_.coef = false;
         pm_.cs = cs;
     }
 }
 
-void EngineBase::transport_retract(SVec* tg, SVec* td, const SVec* g, const SVec* d, SVec* u, double ag,
-                                   double bg, double cg, double ad, double bd, double cd, double cs, double tau) {
+void EngineBase::transport_retract(SVec* tg, SVec* td, const SVec* g, const SVec* d, SVec* u, double tau, int lnq) {
     const PhysMemo keep = pm_;
     state_written(tg);
     state_written(td);
     state_written(u);
     SpecGeom geo = geom(b2);
     const long nt = 3 * geo.ncomp;
+    if (!d_coef_) d_coef_ = (double*)dev_alloc(2 * sizeof(double));
+    const TransportArgs a{d_results, lnq, NAN_SLOT, P.q, P.B, tau, d_coef_};
     cudaEvent_t ev = prof_mark();
     if (state32_)
         spec_transport_kernel<float2><<<grid_for(nt, 256), 256, 0, stream>>>(
-            nt, (const float2*)g, (const float2*)d, (float2*)u, (float2*)tg, (float2*)td, ag, bg, cg, ad, bd, cd, cs,
-            cs * tau);
+            nt, (const float2*)g, (const float2*)d, (float2*)u, (float2*)tg, (float2*)td, a);
     else
         spec_transport_kernel<double2><<<grid_for(nt, 256), 256, 0, stream>>>(
-            nt, (const double2*)g, (const double2*)d, (double2*)u, (double2*)tg, (double2*)td, ag, bg, cg, ad, bd, cd,
-            cs, cs * tau);
+            nt, (const double2*)g, (const double2*)d, (double2*)u, (double2*)tg, (double2*)td, a);
     launched("spec_lincomb", (double)sv_elem() * nt * 6, ev);
     if (keep.tr && keep.u == (const void*)u && keep.d == (const void*)d && keep.tau == tau) {
         pm_ = keep;
         pm_.u = nullptr;  // the fields describe the old u, no longer stored
         pm_.ls = false;
         pm_.next = u;
-        pm_.cs = cs;
+        pm_.coef = true;
     }
 }
 
@@ -335,7 +337,7 @@ void EngineBase::hilbert_leray(SVec* f, double order, double scale) {
     launched("spec_hilbert_leray", 6.0 * sv_elem() * g.ncomp, ev);
 }
 
-void EngineBase::hilbert_leray_pair_dots(SVec* f1, SVec* f2, double order, double s2, double out[2]) {
+void EngineBase::hilbert_leray_pair_dots(SVec* f1, SVec* f2, double order, int lqq) {
     state_written(f1);
     state_written(f2);
     SpecGeom g = geom(b2);
@@ -345,31 +347,30 @@ void EngineBase::hilbert_leray_pair_dots(SVec* f1, SVec* f2, double order, doubl
     ensure_partials((long)grid * 2);
     cudaEvent_t ev = prof_mark();
     if (state32_)
-        spec_hilbert_leray_pair_dot_kernel<float2><<<grid, 128, 0, stream>>>(g, (float2*)f1, 1.0, (float2*)f2, s2, t,
-                                                                              hw, d_partials);
+        spec_hilbert_leray_pair_dot_kernel<float2><<<grid, 128, 0, stream>>>(
+            g, (float2*)f1, 1.0, (float2*)f2, d_results + lqq, P.q, t, hw, d_partials);
     else
-        spec_hilbert_leray_pair_dot_kernel<double2><<<grid, 128, 0, stream>>>(g, (double2*)f1, 1.0, (double2*)f2,
-                                                                               s2, t, hw, d_partials);
+        spec_hilbert_leray_pair_dot_kernel<double2><<<grid, 128, 0, stream>>>(
+            g, (double2*)f1, 1.0, (double2*)f2, d_results + lqq, P.q, t, hw, d_partials);
     launched("spec_hilbert_leray", 2 * 6.0 * sv_elem() * g.ncomp, ev);
-    finalize(grid, 2, 1.0, 200);
-    fetch_results();
-    out[0] = h_results[200];
-    out[1] = h_results[201];
+    finalize(grid, 2, 1.0, RS_CC);
 }
 
-void EngineBase::direction(SVec* gv, double sg, SVec* d, double beta, const SVec* td) {
+void EngineBase::direction(SVec* gv, SVec* d, const SVec* td, const SVec* u, bool normalize, bool conjugate,
+                           bool reset) {
     state_written(gv);
     state_written(d);
     SpecGeom g = geom(b2);
     const long nt = 3 * g.ncomp;
+    const DirectionArgs a{d_results, normalize ? 1 : 0, conjugate ? 1 : 0, reset ? 1 : 0, g.ncomp};
     cudaEvent_t ev = prof_mark();
     if (state32_)
-        spec_direction_kernel<float2><<<grid_for(nt, 256), 256, 0, stream>>>(nt, (float2*)gv, sg, (float2*)d,
-                                                                            td ? beta : 0.0, (const float2*)td);
+        spec_direction_kernel<float2><<<grid_for(nt, 256), 256, 0, stream>>>(nt, (float2*)gv, (float2*)d,
+                                                                            (const float2*)td, (const float2*)u, a);
     else
-        spec_direction_kernel<double2><<<grid_for(nt, 256), 256, 0, stream>>>(nt, (double2*)gv, sg, (double2*)d,
-                                                                             td ? beta : 0.0, (const double2*)td);
-    launched("spec_lincomb", (double)sv_elem() * nt * (3 + (td ? 1 : 0)), ev);
+        spec_direction_kernel<double2><<<grid_for(nt, 256), 256, 0, stream>>>(nt, (double2*)gv, (double2*)d,
+                                                                             (const double2*)td, (const double2*)u, a);
+    launched("spec_lincomb", (double)sv_elem() * nt * (conjugate && !reset ? 4 : 3), ev);
 }
 
 // ---- spectral inner products ----
@@ -422,8 +423,13 @@ constexpr unsigned long long DOT_CG = dot_pp(0, 5, 0) | dot_pp(1, 5, 5) | dot_pp
                                       dot_ax(5, 0);
 constexpr unsigned long long DOT_TRANSPORT = dot_pp(0, 0, 1) | dot_pp(1, 0, 2);
 
-void EngineBase::dots(const SpecDotPair* pairs, int np, double* out, SVec* ax_out, const SVec* ax_x, double ax_a,
-                      const SVec* ax_y) {
+void EngineBase::dots(const SpecDotPair* pairs, int np, double* out) {
+    dots_async(pairs, np);
+    fetch_results();
+    for (int i = 0; i < np; ++i) out[i] = h_results[RS_IP + i];
+}
+
+void EngineBase::dots_async(const SpecDotPair* pairs, int np, SVec* ax_out, const SVec* ax_x, const SVec* ax_y) {
     if (np < 1 || np > 8) throw CudaError("dots: 1 to 8 pairs per call", MLQ_ERR_BADARG);
     SpecDotArgs a;
     a.g = geom(b2);
@@ -434,7 +440,8 @@ void EngineBase::dots(const SpecDotPair* pairs, int np, double* out, SVec* ax_ou
         a.ax_out = ax_out;
         a.ax_x = ax_x;
         a.ax_y = ax_y;
-        a.ax_a = ax_a;
+        a.ax_cc = d_results + RS_CC;
+        a.ax_alpha = d_results + RS_ALPHA;
     }
     bool need_h = false;
     for (int i = 0; i < np; ++i) need_h |= pairs[i].kind == 1;
@@ -500,9 +507,7 @@ void EngineBase::dots(const SpecDotPair* pairs, int np, double* out, SVec* ax_ou
     const bool out_read = ax_out && (ax_out == ax_x || ax_out == ax_y);
     const int nread = nv - ((a.ax_last && !out_read) ? 1 : 0);
     launched("spec_dot", 3.0 * sv_elem() * a.g.ncomp * (nread + (ax_out ? 1 : 0)), ev);
-    finalize(grid, 8, 1.0, 200);
-    fetch_results();
-    for (int i = 0; i < np; ++i) out[i] = h_results[200 + i];
+    finalize(grid, 8, 1.0, RS_IP);
 }
 
 void EngineBase::zeroth(const SVec* f, double out[3]) {

@@ -70,7 +70,7 @@ class EngineBase {
     // result slot the forward transforms set when they meet a non-finite
     // value; fetch_results() turns it into MLQ_ERR_NAN
     static constexpr int NAN_SLOT = NRES - 1;
-    double h_results[NRES];
+    double* h_results = nullptr;  // pinned
     void fetch_results();  // sync + copy all slots; throws MLQ_ERR_NAN if a NaN was seen
 
     // FP64 state spectra (3 components each) of band b2
@@ -111,12 +111,16 @@ class EngineBase {
     // (kinds 2-4 read only a)
     // pairs' inner products; optionally ax_out <- ax_x + ax_a ax_y first, in
     // the same pass (the pairs may name ax_out)
-    void dots(const SpecDotPair* pairs, int np, double* out, SVec* ax_out = nullptr,
-              const SVec* ax_x = nullptr, double ax_a = 0.0, const SVec* ax_y = nullptr);
-    // hilbert_leray of f1 (scale 1) and f2 (scale s2), then out = {<f2, f1>_H, <f2, f2>_H}
-    void hilbert_leray_pair_dots(SVec* f1, SVec* f2, double order, double s2, double out[2]);
-    // g <- sg g, d <- g + beta td (td null: d <- g)
-    void direction(SVec* g, double sg, SVec* d, double beta, const SVec* td);
+    void dots(const SpecDotPair* pairs, int np, double* out);
+    // the same, left in the results (RS_IP ...) on the device; with ax_out,
+    // ax_out <- ax_x - alpha ax_y, alpha from the results (RS_CC)
+    void dots_async(const SpecDotPair* pairs, int np, SVec* ax_out = nullptr, const SVec* ax_x = nullptr,
+                    const SVec* ax_y = nullptr);
+    // hilbert_leray of f1 and of f2 scaled by ||u||_q^{1-q} (||u||_q^q in
+    // result slot lqq), then <f2, f1>_H, <f2, f2>_H in the results (RS_CC)
+    void hilbert_leray_pair_dots(SVec* f1, SVec* f2, double order, int lqq);
+    // g <- sg g, d <- g + beta td, sg and beta from the products in RS_IP
+    void direction(SVec* g, SVec* d, const SVec* td, const SVec* u, bool normalize, bool conjugate, bool reset);
     void zeroth(const SVec* f, double out[3]);
 
     // ---- diagnostics (maxdLpdt.f90:263-299, optimization.f90:119-123, 377-384) ----
@@ -156,6 +160,7 @@ class EngineBase {
         const void* next = nullptr;
         int iu = -1, idu = -1;
         bool ls = false, tr = false, sac = false;
+        bool coef = false;  // d_coef_ holds cs and tau already
         double tau = 0.0, cs = 0.0;
     } pm_;
     // the state spectrum whose S = P2(|u|^2) the physical field 18 and a work
@@ -169,10 +174,11 @@ class EngineBase {
     // u <- cs (u + tau d), keeping the transport's physical fields of
     // u + tau d for the next gradient program
     void retract(SVec* u, double cs, double tau, const SVec* d);
-    // the vector transport's outputs tg = ag g + bg u + cg d, td = ad d + bd u
-    // + cd d and then the retraction u <- cs (u + tau d), in one pass
-    void transport_retract(SVec* tg, SVec* td, const SVec* g, const SVec* d, SVec* u, double ag,
-                           double bg, double cg, double ad, double bd, double cd, double cs, double tau);
+    // the vector transports tg of g and td of d and the retraction
+    // u <- (B/||w||_q) w, w = u + tau d, in one pass (spec_transport_kernel);
+    // ||w||_q^q in result slot lnq
+    void transport_retract(SVec* tg, SVec* td, const SVec* g, const SVec* d, SVec* u, double tau, int lnq);
+    double* d_coef_ = nullptr;  // cs, tau of the retraction (read by a captured launch)
     void ensure_partials(long n);
     // Count a launch and surface launch-configuration errors immediately.
     // With profiling on, `a` is the event recorded before the launch; the
@@ -414,12 +420,17 @@ class Engine : public EngineBase {
     // dealiased |u|^{q-2} u spectra (for calcConstraintDerivativeL2) into
     // c (FP64, may be null) and ||u||_q^q.
     void grad_l2(const SVec* u, SVec* v, SVec* c, double* lqq);
+    // the same without a fetch; returns the result slot of ||u||_q^q
+    int grad_l2_async(const SVec* u, SVec* v, SVec* c, bool want_lq);
     void grad_l2_body(const SVec* u, SVec* v, SVec* c, bool want_lq, bool from_retraction);
     int grad_lq_slot_ = 0;
     // vectorTransport pieces at w = u + tau*d: ir[i] = <P2(|w|^{q-2} w), xi_i>,
     // returns ||w||_q^q.
     double transport_pieces(const SVec* u, const SVec* d, double tau, const SVec* const* xi, int nxi,
                             double* ir);
+    // the same for up to 6 xi without a fetch: ir in RS_IP ..., returns the
+    // result slot of ||w||_q^q
+    int transport_async(const SVec* u, const SVec* d, double tau, const SVec* const* xi, int nxi);
     double lq_pow(const SVec* u, const SVec* d, double tau);  // ||u + tau d||_q^q
     // |u|^k physical (calc_uk) of the state u, into phys index dst
     void calc_uk(const SVec* u, double k, int dst);
@@ -530,7 +541,6 @@ class Engine : public EngineBase {
     void widen_to(const Band& b);
 
     SVec* c_tmp_ = nullptr;  // FP64 spectra of P2(|w|^{q-2} w) for the transport
-    double* d_coef_ = nullptr;  // cs, tau of the retraction (read by a captured launch)
     void phys_written(int idx);  // clears the physical-field memo when it covers idx
     bool w_from_memo(const SVec* u, const SVec* d, double tau);
     bool ls_clamp_free(double tau);  // S(tau) >= 0 at every point (the interval, else one check)

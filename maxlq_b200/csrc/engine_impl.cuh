@@ -1958,11 +1958,11 @@ void Engine<T>::pointwise_R(const SVec* u, double* host) {
 // terms is a dealiased product; their sum is dealiased once (the projection
 // is linear), the fifth term nu Lap P2(|u|^{q-2}u) is added in the spectrum.
 template <typename T>
-void Engine<T>::grad_l2(const SVec* u, SVec* v, SVec* c, double* lqq) {
+int Engine<T>::grad_l2_async(const SVec* u, SVec* v, SVec* c, bool want_lq) {
     if (!c) throw CudaError("grad_l2 needs a spectrum buffer for |u|^{q-2}u", MLQ_ERR_BADARG);
     // u = cs w from the last line search's transport: u and grad u pointwise
     const bool rt = !slab_ && reuse_on_ && pm_.tr && pm_.next == (const void*)u;
-    if (rt) {
+    if (rt && !pm_.coef) {
         if (!d_coef_) d_coef_ = (double*)dev_alloc(2 * sizeof(double));
         const double h[2] = {pm_.cs, pm_.tau};
         MLQ_CUDA(cudaMemcpyAsync(d_coef_, h, sizeof(h), cudaMemcpyHostToDevice, stream));
@@ -1970,14 +1970,20 @@ void Engine<T>::grad_l2(const SVec* u, SVec* v, SVec* c, double* lqq) {
     // the same launches every CG iteration: a CUDA graph after the first two
     // (one per path: the physical fields the retraction reads are in the key)
     as_graph(rt ? (pm_.sac ? "grad_l2_rts" : "grad_l2_rt") : "grad_l2",
-             {u, v, c, lqq ? (const void*)v : nullptr, rt ? (const void*)phys(pm_.idu) : nullptr},
-             [&] { grad_l2_body(u, v, c, lqq != nullptr, rt); });
+             {u, v, c, want_lq ? (const void*)v : nullptr, rt ? (const void*)phys(pm_.idu) : nullptr},
+             [&] { grad_l2_body(u, v, c, want_lq, rt); });
     pm_ = PhysMemo{};        // a replayed graph runs no host code: clear here
     if (!slab_) pu_of_ = u;  // PU, PD hold u and grad u until the next program
     ws_of_ = slab_ ? nullptr : (const void*)u;  // and PS, WS its S
+    return grad_lq_slot_;
+}
+
+template <typename T>
+void Engine<T>::grad_l2(const SVec* u, SVec* v, SVec* c, double* lqq) {
+    const int slot = grad_l2_async(u, v, c, lqq != nullptr);
     if (lqq) {
         fetch_results();
-        *lqq = h_results[grad_lq_slot_];
+        *lqq = h_results[slot];
     }
 }
 
@@ -2240,6 +2246,15 @@ double Engine<T>::lq_pow(const SVec* u, const SVec* d, double tau) {
 template <typename T>
 double Engine<T>::transport_pieces(const SVec* u, const SVec* d, double tau, const SVec* const* xi,
                                    int nxi, double* ir) {
+    const int slot = transport_async(u, d, tau, xi, nxi);
+    fetch_results();
+    for (int i = 0; i < nxi; ++i) ir[i] = h_results[RS_IP + i];
+    return h_results[slot];
+}
+
+template <typename T>
+int Engine<T>::transport_async(const SVec* u, const SVec* d, double tau, const SVec* const* xi, int nxi) {
+    if (nxi < 1 || nxi > 6) throw CudaError("transport: 1 to 6 vectors", MLQ_ERR_BADARG);
     pu_of_ = nullptr;
     const long nc = spec_ncomp();
     const double q = P.q;
@@ -2300,24 +2315,18 @@ double Engine<T>::transport_pieces(const SVec* u, const SVec* d, double tau, con
         if (a2.kind != PowField::ONE) throw CudaError("vectorTransport with 2 < q < 2+eps", MLQ_ERR_BADARG);
         lincomb(cbuf, 1.0, u, d ? tau : 0.0, d, 0.0, nullptr);
     }
-    double lqq;
+    int slot = 0;
     if (ah.kind == PowField::RAW || ah.spec < 0) {
-        pointwise(FSqRed{}, {ah.phys}, {}, 20);
-        fetch_results();
-        lqq = h_results[20];
+        slot = 20;
+        pointwise(FSqRed{}, {ah.phys}, {}, slot);
     } else {
         ensure_p2_spec(ah);
-        sdots(*this, {{wspec(ah.spec), wspec(ah.spec)}}, 0);
-        fetch_results();
-        lqq = h_results[0];
+        sdots(*this, {{wspec(ah.spec), wspec(ah.spec)}}, slot);
     }
-    for (int k = 0; k < nxi; k += 6) {
-        SpecDotPair pr[6];
-        const int m = std::min(6, nxi - k);
-        for (int i = 0; i < m; ++i) pr[i] = SpecDotPair{cbuf, xi[k + i], 0};
-        dots(pr, m, ir + k);
-    }
-    return lqq;
+    SpecDotPair pr[6];
+    for (int i = 0; i < nxi; ++i) pr[i] = SpecDotPair{cbuf, xi[i], 0};
+    dots_async(pr, nxi);
+    return slot;
 }
 
 // calc_uk (function_ops.f90:2324-2343) of the state u into phys(dst)

@@ -617,6 +617,38 @@ __global__ void __launch_bounds__(256) zinv_kernel(ZInvArgs<T> a) {
 // ----------------------------------------------------------------------------
 // Spectral-state kernels on pruned FP64 vector spectra [3][nb][nb][nx].
 // ----------------------------------------------------------------------------
+
+// ---- scalars of the CG update -------------------------------------------------
+// The kernels of an iteration read the sums that their factors come from in
+// the result slots on the device, so that the host fetches once per line
+// search and once at the iteration's end instead of after every reduction (a
+// fetch costs some 12 us with the launches that wait for it: 9 of them and 6
+// scalar copies took a quarter of an iteration at 64^3).  The thread that
+// computes a factor for the host's record leaves it in a slot of its own.
+enum : int {
+    RS_IP = 200,     // 200..207: the products of the update (dots)
+    RS_CC = 216,     // 216, 217: <c, g>, <c, c>
+    RS_ALPHA = 224,  // alpha, sg, beta of this iteration
+    RS_SG = 225,
+    RS_BETA = 226,
+    RS_MEAN = 240,   // 240..242 d, 243..245 u: the k = 0 coefficients
+};
+// sg, beta from the products (optimization.f90:213, 226-238)
+enum : int { IP_GC, IP_GDIV, IP_GG, IP_UU, IP_GTG, IP_G0G0, IP_GTD, IP_TDTD };
+__device__ __forceinline__ void cg_direction_factors(const double* ip, int normalize, int conjugate, int reset,
+                                                     double& sg, double& beta) {
+    sg = normalize ? sqrt(ip[IP_UU] / ip[IP_GG]) : 1.0;  // 213
+    beta = 0.0;
+    if (conjugate) {
+        beta = sg * sg * ip[IP_GG] - sg * ip[IP_GTG];  // <g', g' - T g0> (226)
+        const double g0n = ip[IP_G0G0];                // 227
+        if (g0n < MACH_EPSILON || beta < MACH_EPSILON)
+            beta = 0.0;
+        else
+            beta = beta / g0n;
+        if (reset) beta = 0.0;  // 235-238
+    }
+}
 struct SpecGeom {
     int n, nx, nb;
     Band band;
@@ -686,15 +718,37 @@ __global__ void spec_poly3_kernel(C* out, const C* a, const C* b, const C* c, lo
 }
 
 // The vector transport's two outputs and the retraction in one pass over the
-// state (function_ops.f90:1716-1768 with optimization.f90:324-338):
-//   tg = ag g + bg u + cg d,  td = ad d + bd u + cd d,  u <- cs u + ct d
+// state (function_ops.f90:1716-1768 with optimization.f90:324-338), with
+// w = u + tau d, ln = ||w||_q, ir_x = <P2(|w|^{q-2} w), x>:
+//   T x = (B/ln) (x - ln^-q ir_x w) for x = g, d;  u <- (B/ln) w
+// lnq = ln^q and ir_g, ir_d are read from the results; nothing is written when
+// a NaN was flagged on the way.  coef <- (B/ln, tau) for the next gradient.
+struct TransportArgs {
+    const double* results;
+    int lnq_slot, nan_slot;  // ir in RS_IP, RS_IP + 1
+    double q, B, tau;
+    double* coef;
+};
 template <typename V>
-__global__ void spec_transport_kernel(long nt, const V* g, const V* d, V* u, V* tg, V* td, double ag, double bg,
-                                      double cg, double ad, double bd, double cd, double cs, double ct) {
+__global__ void spec_transport_kernel(long nt, const V* g, const V* d, V* u, V* tg, V* td, TransportArgs a) {
+    __shared__ double f[3];
+    if (threadIdx.x == 0) {
+        const double ln = pow(a.results[a.lnq_slot], 1.0 / a.q), cs = a.B / ln, fq = pow(ln, -a.q);
+        f[0] = cs;
+        f[1] = -cs * fq * a.results[RS_IP];
+        f[2] = -cs * fq * a.results[RS_IP + 1];
+        if (blockIdx.x == 0) {
+            a.coef[0] = cs;
+            a.coef[1] = a.tau;
+        }
+    }
+    __syncthreads();
+    if (a.results[a.nan_slot] != 0.0) return;
+    const double cs = f[0], bg = f[1], bd = f[2], cg = bg * a.tau, cd = bd * a.tau, ct = cs * a.tau;
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < nt; i += (long)gridDim.x * blockDim.x) {
         const double2 gv = ldv(g, i), dv = ldv(d, i), uv = ldv(u, i);
-        stv(tg, i, make_double2(ag * gv.x + bg * uv.x + cg * dv.x, ag * gv.y + bg * uv.y + cg * dv.y));
-        stv(td, i, make_double2(ad * dv.x + bd * uv.x + cd * dv.x, ad * dv.y + bd * uv.y + cd * dv.y));
+        stv(tg, i, make_double2(cs * gv.x + bg * uv.x + cg * dv.x, cs * gv.y + bg * uv.y + cg * dv.y));
+        stv(td, i, make_double2(cs * dv.x + bd * uv.x + cd * dv.x, cs * dv.y + bd * uv.y + cd * dv.y));
         stv(u, i, make_double2(cs * uv.x + ct * dv.x, cs * uv.y + ct * dv.y));
     }
 }
@@ -767,13 +821,18 @@ __global__ void spec_hilbert_leray_kernel(SpecGeom g, V* f, const double* __rest
 }
 
 // Hilbert gradient + Leray projection of two fields (f1 scaled by s1, f2 by
-// s2) and, on the results, the H inner products <f2, f1> and <f2, f2> (the
+// ||u||_q^{1-q}, from ||u||_q^q at lqq) and, on the results, the H inner products <f2, f1> and <f2, f2> (the
 // weights of spec_dot_kernel's kind 1) as per-block partials [block][2]
 template <typename V>
 __global__ void __launch_bounds__(128) spec_hilbert_leray_pair_dot_kernel(SpecGeom g, V* f1, double s1, V* f2,
-                                                                       double s2, const double* __restrict__ htab,
+                                                                       const double* __restrict__ lqq, double q,
+                                                                       const double* __restrict__ htab,
                                                                        const double* __restrict__ hwtab,
                                                                        double* partials) {
+    __shared__ double s2sh;  // ||u||_q^{1-q} from ||u||_q^q
+    if (threadIdx.x == 0) s2sh = pow(pow(*lqq, 1.0 / q), 1.0 - q);
+    __syncthreads();
+    const double s2 = s2sh;
     const double twopi = 2.0 * 3.14159265358979311600;
     const int nrows = g.nb * g.nb;
     double acc[2] = {0.0, 0.0};
@@ -811,20 +870,38 @@ __global__ void __launch_bounds__(128) spec_hilbert_leray_pair_dot_kernel(SpecGe
 }
 
 // The search direction from the projected gradient: g <- sg g, then
-// d <- g + beta td (td may be null: d <- g)
+// d <- g + beta td, with sg and beta from the update's products.  Leaves them
+// and the k = 0 coefficients of d and u in the results.
+struct DirectionArgs {
+    double* results;
+    int normalize, conjugate, reset;
+    long ncomp;
+};
 template <typename V>
-__global__ void spec_direction_kernel(long nt, V* g, double sg, V* d, double beta, const V* td) {
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < nt; i += (long)gridDim.x * blockDim.x) {
+__global__ void spec_direction_kernel(long nt, V* g, V* d, const V* td, const V* u, DirectionArgs a) {
+    double sg, beta;
+    cg_direction_factors(a.results + RS_IP, a.normalize, a.conjugate, a.reset, sg, beta);
+    const long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i0 == 0) {
+        a.results[RS_SG] = sg;
+        a.results[RS_BETA] = beta;
+    }
+    for (long i = i0; i < nt; i += (long)gridDim.x * blockDim.x) {
         double2 v = ldv(g, i);
         v.x *= sg;
         v.y *= sg;
         stv(g, i, v);
-        if (td) {
+        if (beta != 0.0) {
             const double2 w = ldv(td, i);
             v.x += beta * w.x;
             v.y += beta * w.y;
         }
         stv(d, i, v);
+        if (i % a.ncomp == 0) {
+            const int c = (int)(i / a.ncomp);
+            a.results[RS_MEAN + c] = rndv<V>(v).x;
+            a.results[RS_MEAN + 3 + c] = ldv(u, i).x;
+        }
     }
 }
 
@@ -841,12 +918,13 @@ struct SpecDotArgs {
     SpecGeom g;
     SpecDotPair pr[8];
     int npairs;
-    // optional ax_out <- ax_x + ax_a ax_y before the products (the pairs may
+    // optional ax_out <- ax_x - alpha ax_y before the products (the pairs may
     // read ax_out: each element is updated by the thread that then reads it)
     void* ax_out = nullptr;
     const void* ax_x = nullptr;
     const void* ax_y = nullptr;
-    double ax_a = 0.0;
+    const double* ax_cc = nullptr;  // ax_a = -alpha, alpha = ax_cc[0] / ax_cc[1]
+    double* ax_alpha = nullptr;     // alpha is left here
     // the distinct vectors of the pass for spec_dot_fixed_kernel, ax_out
     // last when the pass reads it (ax_last)
     const void* vec[8];
@@ -885,12 +963,20 @@ __device__ __forceinline__ double dot_term(int kind, const double2 (&u)[3], cons
     return kind == 1 ? hw * s : s;
 }
 
+__device__ __forceinline__ double dot_ax_factor(const SpecDotArgs& a) {
+    if (!a.ax_out) return 0.0;
+    const double alpha = a.ax_cc[0] / a.ax_cc[1];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.ax_alpha = alpha;
+    return -alpha;
+}
+
 // Up to 8 inner products with every pair's vectors loaded per pair (any
 // pattern of operands).  One warp per row, each lane one mode at a time.
 template <typename V>
 __global__ void __launch_bounds__(RED_THREADS) spec_dot_kernel(SpecDotArgs a) {
     double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     const SpecGeom& g = a.g;
+    const double ax_a = dot_ax_factor(a);
     const double twopi = 2.0 * 3.14159265358979311600;
     const int nrows = g.nb * g.nb;
     const int lane = threadIdx.x & 31, wrow = threadIdx.x >> 5, rows_per = blockDim.x >> 5;
@@ -910,7 +996,7 @@ __global__ void __launch_bounds__(RED_THREADS) spec_dot_kernel(SpecDotArgs a) {
                 for (int c = 0; c < 3; ++c) {
                     const long k = c * g.ncomp + i;
                     const double2 x = ldv((const V*)a.ax_x, k), y = ldv((const V*)a.ax_y, k);
-                    stv((V*)a.ax_out, k, make_double2(x.x + a.ax_a * y.x, x.y + a.ax_a * y.y));
+                    stv((V*)a.ax_out, k, make_double2(x.x + ax_a * y.x, x.y + ax_a * y.y));
                 }
             }
             // unrolled to the bound of 8 so that acc stays in registers
@@ -933,12 +1019,13 @@ __global__ void __launch_bounds__(RED_THREADS) spec_dot_kernel(SpecDotArgs a) {
 // The same products for a pattern of operands fixed at compile time: the NV
 // distinct vectors are loaded once per mode, pair p reads vec[(PAT >> 6p) & 7]
 // and vec[(PAT >> (6p + 3)) & 7], and the optional update reads
-// vec[(PAT >> 48) & 7] + ax_a vec[(PAT >> 51) & 7] and writes ax_out (which
+// vec[(PAT >> 48) & 7] - alpha vec[(PAT >> 51) & 7] and writes ax_out (which
 // replaces vec[NV - 1] when ax_last).
 template <typename V, int NV, int NP, unsigned long long PAT>
 __global__ void __launch_bounds__(RED_THREADS) spec_dot_fixed_kernel(SpecDotArgs a) {
     double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     const SpecGeom& g = a.g;
+    const double ax_a = dot_ax_factor(a);
     const double twopi = 2.0 * 3.14159265358979311600;
     const int nrows = g.nb * g.nb;
     constexpr int XI = (int)((PAT >> 48) & 7), YI = (int)((PAT >> 51) & 7);
@@ -967,7 +1054,7 @@ __global__ void __launch_bounds__(RED_THREADS) spec_dot_fixed_kernel(SpecDotArgs
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     const double2 nv =
-                        rndv<V>(make_double2(x[XI][c].x + a.ax_a * x[YI][c].x, x[XI][c].y + a.ax_a * x[YI][c].y));
+                        rndv<V>(make_double2(x[XI][c].x + ax_a * x[YI][c].x, x[XI][c].y + ax_a * x[YI][c].y));
                     stv((V*)a.ax_out, c * g.ncomp + i, nv);
                     if (a.ax_last) x[NV - 1][c] = nv;
                 }

@@ -194,9 +194,11 @@ class Solver : public SolverBase {
         }
         MLQ_CUDA(cudaEventRecord(ev0_, e.stream));
     }
-    double iter_clock_stop() {
+    void iter_clock_stop() {
         MLQ_CUDA(cudaEventRecord(ev1_, e.stream));
-        MLQ_CUDA(cudaEventSynchronize(ev1_));
+        e.fetch_results();
+    }
+    double iter_seconds() {
         float ms = 0.f;
         MLQ_CUDA(cudaEventElapsedTime(&ms, ev0_, ev1_));
         return ms * 1e-3;
@@ -211,62 +213,54 @@ class Solver : public SolverBase {
         trials.clear();
         const double qq = q(), Bc = B();
         const double s = (3.0 / 2.0) - (1.0 / qq);  // 150
+        if (!e.P.use_tangential_gradient) throw CudaError("useTangentialGradient=.false. is not supported",
+                                                          MLQ_ERR_BADARG);
         SVec* g1 = gu1;
-        double lqq_u = 0;
-        e.grad_l2(u, g1, c, &lqq_u);  // 146
+        // The update up to the direction runs without the host: each kernel
+        // reads the sums that its factors come from (RS_CC, RS_IP) on the
+        // device, and the host reads them with the line search's first result.
+        const int lqq_u = e.grad_l2_async(u, g1, c, true);  // 146
         // Hilbert gradient of g (151, 153) and of the normal of the tangent
         // space ||u||_q^{1-q} P2(|u|^{q-2} u) (162, 164, 169), with <c, g>
         // and <c, c> (170-171) in the same pass
-        const double unorm = std::pow(lqq_u, 1.0 / qq);
-        double dd[2];
-        e.hilbert_leray_pair_dots(g1, c, s, std::pow(unorm, 1.0 - qq), dd);
-        const double alpha = dd[0] / dd[1];  // 170-171
-        info.alpha = alpha;
-        if (!e.P.use_tangential_gradient) throw CudaError("useTangentialGradient=.false. is not supported",
-                                                          MLQ_ERR_BADARG);
+        e.hilbert_leray_pair_dots(g1, c, s, lqq_u);
         // Every inner product the rest of the update needs, in one pass.  The
         // reference forms g + c (180-193) and g - T g0 (223-226) and the norm
         // of d1 only to take inner products of them; those are expanded here
         // into products of g, c, u, T g0, g0, T d0 (bilinearity), which
         // saves two state-vector temporaries and four reductions.
-        const double cc = dd[1];  // <c, c>
-        enum { GC, GDIV, GG, UU, GTG, G0G0, GTD, TDTD };
-        double ip[8];
         {
             // gradJproj g <- g - alpha c (177, kept in gu1) in the same pass
             SpecDotPair p[8] = {{g1, c, 1},    {g1, nullptr, 2}, {g1, g1, 1},   {u, u, 1},
                                 {g1, vtg0, 1}, {gu0, gu0, 1},    {g1, vtd0, 1}, {vtd0, vtd0, 1}};
-            e.dots(p, 8, ip, g1, g1, -alpha, c);
+            e.dots_async(p, 8, g1, g1, c);
         }
-        info.ortho_check = std::fabs(ip[GC] / (ip[GG] + 2.0 * ip[GC] + cc));  // <g,c> / <g+c, g+c>
-        info.div_check = ip[GDIV] / ip[GG];
-        double sg = 1.0;  // gradient normalisation (213), applied with d1 below
-        if (e.P.normalize_gradient) sg = std::sqrt(ip[UU] / ip[GG]);
-        const double gg = sg * sg * ip[GG], gtd = sg * ip[GTD];  // <g', g'>, <g', T d0>
-        double beta = 0.0;
-        if (e.P.use_conjugate_gradient) {
-            beta = gg - sg * ip[GTG];  // <g', g' - T g0> (226)
-            const double g0n = ip[G0G0];  // 227
-            if (g0n < MACH_EPSILON || beta < MACH_EPSILON)
-                beta = 0.0;
-            else
-                beta = beta / g0n;
-            if (e.P.reset_momentum_every > 0 && iter % e.P.reset_momentum_every == 0) beta = 0.0;  // 235-238
-            e.direction(g1, sg, d1, beta, vtd0);                                                     // 213, 240
-        } else {
-            e.direction(g1, sg, d1, 0.0, nullptr);
-        }
-        info.beta = beta;
-        info.norm_grad = std::sqrt(gg);
-        info.norm_td0 = std::sqrt(ip[TDTD]);
-        info.norm_d1 = std::sqrt(std::max(0.0, gg + 2.0 * beta * gtd + beta * beta * ip[TDTD]));
-        e.zeroth(d1, info.mean_d1);  // 251
-        e.zeroth(u, info.mean_u);    // 257
+        const bool reset = e.P.reset_momentum_every > 0 && iter % e.P.reset_momentum_every == 0;  // 235-238
+        e.direction(g1, d1, vtd0, u, e.P.normalize_gradient, e.P.use_conjugate_gradient, reset);  // 213, 240
         // line search (269-318)
         double tb[2] = {0, 0};
         int mflag = 0;
         ls_begin(u, d1, tau0);
         double fx = 0, tau1 = 0;
+        // the update's scalars for the record, once the search has fetched them
+        auto record_update = [&] {
+            const double* r = e.h_results;
+            const double *ip = r + RS_IP, cc = r[RS_CC + 1];  // <c, c>
+            const double sg = r[RS_SG], beta = r[RS_BETA];
+            info.alpha = r[RS_ALPHA];
+            info.beta = beta;
+            info.ortho_check = std::fabs(ip[IP_GC] / (ip[IP_GG] + 2.0 * ip[IP_GC] + cc));  // <g,c> / <g+c, g+c>
+            info.div_check = ip[IP_GDIV] / ip[IP_GG];
+            const double gg = sg * sg * ip[IP_GG], gtd = sg * ip[IP_GTD];  // <g', g'>, <g', T d0>
+            info.norm_grad = std::sqrt(gg);
+            info.norm_td0 = std::sqrt(ip[IP_TDTD]);
+            info.norm_d1 = std::sqrt(std::max(0.0, gg + 2.0 * beta * gtd + beta * beta * ip[IP_TDTD]));
+            const double n3 = (double)e.n3;  // unnormalised k=0 coefficients (function_ops.f90:3084-3086)
+            for (int k = 0; k < 3; ++k) {
+                info.mean_d1[k] = r[RS_MEAN + k] * n3;      // 251
+                info.mean_u[k] = r[RS_MEAN + 3 + k] * n3;   // 257
+            }
+        };
         LsOut lo;
         if (ls_ready && e.ls_device_search(Bc, 0.0, tau0, &lo) == 0 && lo.status != LS_ERR_CAP) {
             // mnbrak and Brent ran on the device; one read of the outcome
@@ -288,13 +282,15 @@ class Solver : public SolverBase {
             mnbrak(u, d1, 0.0, tau0, tb, &mflag);
             if (mflag == 0) tau1 = brent(u, d1, tb, &fx);  // 297
         }
+        record_update();
         info.J0 = J0;
         info.mnbrak_flag = mflag;
         if (mflag != 0) {
+            iter_clock_stop();
             info.n_evals = evals_this_iter;
             info.status = mflag == 1 ? MLQ_ERR_MNBRAK_UPHILL : MLQ_ERR_MNBRAK_ITMAX;
             while_flag = 1;
-            info.seconds = iter_clock_stop();
+            info.seconds = iter_seconds();
             return info.status;
         }
         info.tau_a = tb[0];
@@ -307,31 +303,29 @@ class Solver : public SolverBase {
         }
         info.tau = tau1;
         // vector transport of gu1 and d1 to the new point (324-328)
-        double ir[2];
         const SVec* xi[2] = {g1, d1};
         ls_ready = lsg_ready = false;
-        double lqw;
-        if (e.P.use_riemannian_geometry)
-            lqw = e.transport_pieces(u, d1, tau1, xi, 2, ir);
-        else
-            lqw = e.lq_pow(u, d1, tau1);
-        const double ln = std::pow(lqw, 1.0 / qq);
         // R at the retracted point from the accepted trial (homogeneity), as
         // eval_J(Uvec, "maxdLqdt") after rescaleLqNorm (344-349)
         const Trial tr = trial(u, d1, tau1);
+        int lnq = 0;
+        double ln = 0.0;
+        if (e.P.use_riemannian_geometry)
+            lnq = e.transport_async(u, d1, tau1, xi, 2);
+        else
+            ln = std::pow(e.lq_pow(u, d1, tau1), 1.0 / qq);
         const double cs = Bc / std::pow(tr.lqq, 1.0 / qq);
         const double R12n = std::pow(cs, qq) * tr.R[1], R3n = std::pow(cs, qq + 1.0) * tr.R[2];
         if (e.P.use_riemannian_geometry) {
             // transported gradient and direction (324-328), then u <- (B/ln) w
-            const double f = std::pow(ln, -qq);
-            e.transport_retract(vtg0, vtd0, g1, d1, u, Bc / ln, -Bc / ln * f * ir[0], -Bc / ln * f * ir[0] * tau1,
-                                Bc / ln, -Bc / ln * f * ir[1], -Bc / ln * f * ir[1] * tau1, Bc / ln, tau1);
+            e.transport_retract(vtg0, vtd0, g1, d1, u, tau1, lnq);
         } else {
             e.lincomb(vtg0, 1.0, g1);
             e.lincomb(vtd0, 1.0, d1);
             e.retract(u, Bc / ln, tau1, d1);
         }
         trials.clear();
+        iter_clock_stop();  // with the fetch: a NaN in the transport is reported before the new state counts
         const double J1 = R12n + R3n;
         const double deltaJ = (J1 - J0) / std::fabs(J0);
         info.J1 = J1;
@@ -340,7 +334,7 @@ class Solver : public SolverBase {
         if (deltaJ < -MACH_EPSILON) {  // 351-366
             while_flag = 1;
             info.status = MLQ_ERR_J_DECREASED;
-            info.seconds = iter_clock_stop();
+            info.seconds = iter_seconds();
             return info.status;
         }
         info.u_norm_q = cs * std::pow(tr.lqq, 1.0 / qq);  // ||u||_q after the retraction (421)
@@ -357,7 +351,7 @@ class Solver : public SolverBase {
         for (double r : roll) ssum += r;
         avg_imp = ssum / (double)(iter - start_iter);
         info.status = status;
-        info.seconds = iter_clock_stop();
+        info.seconds = iter_seconds();
         return status;
     }
 
