@@ -475,6 +475,7 @@ __global__ void __launch_bounds__(CShape<N, T>::XTHREADS, 512 / CShape<N, T>::XT
         tw.tab = stw;
     }
     const cpx<T> wt = twN[t];  // W_N^t
+    pdl_begin<(N <= 64)>();
     const int nx_in = a.nx_in;
     const int px = a.px ? a.px : nx_in;  // row pitch of xs
     const cpx<T>* __restrict__ src0 = a.in[blockIdx.y];
@@ -569,6 +570,7 @@ __global__ void __launch_bounds__(CShape<N, T>::XTHREADS, xfwd_minb<F>() * 256 /
         tw.tab = stw;
     }
     const cpx<T> wt = twN[t];  // W_N^t
+    pdl_begin<(N <= 64)>();
     const int nx = a.nx;
     const int px = a.px ? a.px : nx;  // row pitch of xs
     const int src_lane = (TPL - t) & (TPL - 1);
@@ -656,6 +658,7 @@ __global__ void __launch_bounds__(YShape<N, T, V>::YTHREADS, YShape<N, T, V>::YM
     __syncthreads();
     const int l = threadIdx.x % TX, t = threadIdx.x / TX;
     const YTw<N, E, T, S::TWREG> tw(stw, twN, t);
+    pdl_begin<(N <= 64)>();
     const ColMap<TX> map{l};
     const int nx = a.nx, nb = a.band.nb;
     const int px = a.px ? a.px : nx;  // row pitch of xs and ys
@@ -1034,6 +1037,7 @@ __global__ void __launch_bounds__(YShape<N, T, V>::YTHREADS, YShape<N, T, V>::YM
     __syncthreads();
     const int l = threadIdx.x % TX, t = threadIdx.x / TX;
     const YTw<N, E, T, S::TWREG> tw(stw, twN, t);
+    pdl_begin<(N <= 64)>();
     const ColMap<TX> map{l};
     const int nx = a.nx, nb = a.band.nb, cut = a.band.cut;
     const int ntile = (nx + TX - 1) / TX;
@@ -1111,6 +1115,7 @@ __global__ void __launch_bounds__(YShape<N, T, V>::YTHREADS, YShape<N, T, V>::YM
     __syncthreads();
     const int l = threadIdx.x % TX, t = threadIdx.x / TX;
     const YTw<N, E, T, S::TWREG> tw(stw, twN, t);
+    pdl_begin<(N <= 64)>();
     const ColMap<TX> map{l};
     const int nx = a.nx, nb = a.band.nb, cut = a.band.cut;
     const int ntile = (nx + TX - 1) / TX;
@@ -1183,6 +1188,7 @@ __global__ void __launch_bounds__(YShape<N, T, V>::YTHREADS, YShape<N, T, V>::YM
     __syncthreads();
     const int l = threadIdx.x % TX, t = threadIdx.x / TX;
     const YTw<N, E, T, S::TWREG> tw(stw, twN, t);
+    pdl_begin<(N <= 64)>();
     const ColMap<TX> map{l};
     const int nx = a.nx, nb = a.band.nb, cut = a.band.cut;
     const int ntile = (nx + TX - 1) / TX;
@@ -1325,6 +1331,7 @@ __global__ void __launch_bounds__(PairShape<N>::THREADS, MINB)
     __syncthreads();
     const int l = threadIdx.x % NP, t = threadIdx.x / NP;
     const TwStage<N, E, float> tw{stw};
+    pdl_begin<(N <= 64)>();
     const int nx = a.nx, nb = a.band.nb;
     const int pp = (a.px ? a.px : nx) / 2;  // row pitch in pairs (the pitch is even)
     const int npair = (nx + 1) / 2;
@@ -1408,6 +1415,7 @@ __global__ void __launch_bounds__(PairShape<N>::THREADS, MINB)
     __syncthreads();
     const int l = threadIdx.x % NP, t = threadIdx.x / NP;
     const TwStage<N, E, float> tw{stw};
+    pdl_begin<(N <= 64)>();
     const int nx = a.nx, nb = a.band.nb, cut = a.band.cut;
     const int pp = (a.px ? a.px : nx) / 2;  // row pitch of the y-stage arrays in pairs
     const int npair = (nx + 1) / 2;
@@ -1486,6 +1494,7 @@ __global__ void __launch_bounds__(PairShape<N>::THREADS, MINB)
     __syncthreads();
     const int l = threadIdx.x % NP, t = threadIdx.x / NP;
     const TwStage<N, E, float> tw{stw};
+    pdl_begin<(N <= 64)>();
     const int nx = a.nx, nb = a.band.nb, cut = a.band.cut;
     const int pp = (a.px ? a.px : nx) / 2;  // row pitch of the y-stage arrays in pairs
     const int npair = (nx + 1) / 2;
@@ -1580,6 +1589,7 @@ __global__ void __launch_bounds__(YShape<N, T, V>::YTHREADS, YShape<N, T, V>::YM
     __syncthreads();
     const G g;
     const TwTab<N, E, T> tw{stw};
+    pdl_begin<(N <= 64)>();
     const RowMap<E> xmap{g.w * S::WPITCH};
     const int nx = a.nx, nb = a.band.nb;
     const int px = a.px ? a.px : nx;  // row pitch of xs and ys
@@ -1654,6 +1664,7 @@ __global__ void __launch_bounds__(YShape<N, T, V>::YTHREADS, YShape<N, T, V>::YM
     __syncthreads();
     const G g;
     const TwTab<N, E, T> tw{stw};
+    pdl_begin<(N <= 64)>();
     const RowMap<E> xmap{g.w * S::WPITCH};
     const int nx = a.nx, nb = a.band.nb, cut = a.band.cut;
     const int ntile = (nx + TX - 1) / TX;
@@ -1738,6 +1749,7 @@ __global__ void __launch_bounds__(YShape<N, T, V>::YTHREADS, YShape<N, T, V>::YM
     __syncthreads();
     const G g;
     const TwTab<N, E, T> tw{stw};
+    pdl_begin<(N <= 64)>();
     const RowMap<E> xmap{g.w * S::WPITCH};
     const int nx = a.nx, nb = a.band.nb, cut = a.band.cut;
     const int ntile = (nx + TX - 1) / TX;

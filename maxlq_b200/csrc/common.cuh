@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <stdexcept>
 #include <string>
+#include <utility>
 
 #include "../../include/maxlq.h"
 
@@ -91,6 +92,42 @@ struct CudaError : std::runtime_error {
     int status;
     CudaError(const std::string& m, int s) : std::runtime_error(m), status(s) {}
 };
+
+// Programmatic dependent launch.  A kernel launched with launch_pdl may start
+// while its predecessor in the stream still drains: everything before
+// pdl_begin (twiddle and wavenumber tables, index arithmetic) overlaps the
+// predecessor's last blocks and the launch gap; pdl_begin waits until the
+// predecessor has completed and its writes are visible.  A kernel calls it
+// once, in every thread, before it touches memory that another kernel of the
+// stream reads or writes.  A CG iteration at q = 4: 64^3 FP64 0.474 -> 0.385
+// ms, 32^3 0.84 -> 0.73, 128^3 FP64 1.59 -> 1.49, 192^3 mixed 3.16 -> 3.03, 256^3 FP64
+// 8.97 -> 8.86, 512^3 mixed unchanged (35.3).
+// EARLY lets the successor start as soon as this kernel's blocks run, instead
+// of as they exit.  64^3 gains from it (0.398 -> 0.380 ms); from 128^3 on it
+// gains nothing and then costs (256^3 FP64 8.86 -> 9.45, 512^3 mixed 35.3 ->
+// 43.5 ms), so the pass kernels take it up to N = 64 and the one-block
+// finalize always.
+template <bool EARLY = false>
+__device__ __forceinline__ void pdl_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if constexpr (EARLY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <class... P, class... A>
+inline cudaError_t launch_pdl(bool on, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                              A&&... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = at;
+    cfg.numAttrs = on ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
 
 #define MLQ_CUDA(call)                                                                          \
     do {                                                                                        \

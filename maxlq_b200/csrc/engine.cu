@@ -58,6 +58,8 @@ EngineBase::EngineBase(const mlq_params& p) : P(p) {
     MLQ_CUDA(cudaStreamSynchronize(stream));
     ensure_partials(1 << 20);
     if (const char* e = std::getenv("MLQ_GRAPHS")) graphs_on_ = std::string(e) != "0";
+    if (const char* e = std::getenv("MLQ_PDL")) pdl_on_ = std::string(e) != "0";
+    pdl_ = pdl_on_;
     if (const char* e = std::getenv("MLQ_REUSE")) reuse_on_ = std::string(e) != "0";
     if (const char* e = std::getenv("MLQ_ZMULTI")) multi_zinv_ = std::string(e) != "0";
 }
@@ -133,7 +135,7 @@ void EngineBase::ensure_partials(long cnt) {
 
 void EngineBase::finalize(int nblocks, int nr, double scale, int dst, bool accumulate) {
     cudaEvent_t ev = prof_mark();
-    finalize_partials_kernel<<<1, FIN_THREADS, 0, stream>>>(d_partials, nblocks, nr, scale, d_results, dst,
+    launch_k(finalize_partials_kernel, 1, FIN_THREADS, 0, d_partials, nblocks, nr, scale, d_results, dst,
                                                            accumulate ? 1 : 0);
     launched("finalize", 8.0 * nblocks * nr, ev);
 }
@@ -218,10 +220,10 @@ void EngineBase::lincomb(SVec* out, double a, const SVec* x, double b, const SVe
     SpecGeom g = geom(b2);
     cudaEvent_t ev = prof_mark();
     if (state32_)
-        spec_lincomb_kernel<float2><<<grid_for(3 * g.ncomp, 256), 256, 0, stream>>>(
+        launch_k(spec_lincomb_kernel<float2>, grid_for(3 * g.ncomp, 256), 256, 0, 
             g, (float2*)out, a, (const float2*)x, b, (const float2*)y, c, (const float2*)z);
     else
-        spec_lincomb_kernel<double2><<<grid_for(3 * g.ncomp, 256), 256, 0, stream>>>(
+        launch_k(spec_lincomb_kernel<double2>, grid_for(3 * g.ncomp, 256), 256, 0, 
             g, (double2*)out, a, (const double2*)x, b, (const double2*)y, c, (const double2*)z);
     launched("spec_lincomb", 3.0 * sv_elem() * g.ncomp * (2 + (y ? 1 : 0) + (z ? 1 : 0)), ev);
 }
@@ -287,10 +289,10 @@ void EngineBase::transport_retract(SVec* tg, SVec* td, const SVec* g, const SVec
     const TransportArgs a{d_results, lnq, NAN_SLOT, P.q, P.B, tau, d_coef_};
     cudaEvent_t ev = prof_mark();
     if (state32_)
-        spec_transport_kernel<float2><<<grid_for(nt, 256), 256, 0, stream>>>(
+        launch_k(spec_transport_kernel<float2>, grid_for(nt, 256), 256, 0, 
             nt, (const float2*)g, (const float2*)d, (float2*)u, (float2*)tg, (float2*)td, a);
     else
-        spec_transport_kernel<double2><<<grid_for(nt, 256), 256, 0, stream>>>(
+        launch_k(spec_transport_kernel<double2>, grid_for(nt, 256), 256, 0, 
             nt, (const double2*)g, (const double2*)d, (double2*)u, (double2*)tg, (double2*)td, a);
     launched("spec_lincomb", (double)sv_elem() * nt * 6, ev);
     if (keep.tr && keep.u == (const void*)u && keep.d == (const void*)d && keep.tau == tau) {
@@ -308,9 +310,9 @@ void EngineBase::hilbert(SVec* f, double order) {
     const double* t = hilbert_table(order);
     cudaEvent_t ev = prof_mark();
     if (state32_)
-        spec_hilbert_leray_kernel<float2><<<spec_rows_grid(g), 128, 0, stream>>>(g, (float2*)f, t, 1.0, 0);
+        launch_k(spec_hilbert_leray_kernel<float2>, spec_rows_grid(g), 128, 0, g, (float2*)f, t, 1.0, 0);
     else
-        spec_hilbert_leray_kernel<double2><<<spec_rows_grid(g), 128, 0, stream>>>(g, (double2*)f, t, 1.0, 0);
+        launch_k(spec_hilbert_leray_kernel<double2>, spec_rows_grid(g), 128, 0, g, (double2*)f, t, 1.0, 0);
     launched("spec_hilbert", 6.0 * sv_elem() * g.ncomp, ev);
 }
 
@@ -319,9 +321,9 @@ void EngineBase::leray(SVec* f) {
     SpecGeom g = geom(b2);
     cudaEvent_t ev = prof_mark();
     if (state32_)
-        spec_hilbert_leray_kernel<float2><<<spec_rows_grid(g), 128, 0, stream>>>(g, (float2*)f, nullptr, 1.0, 1);
+        launch_k(spec_hilbert_leray_kernel<float2>, spec_rows_grid(g), 128, 0, g, (float2*)f, nullptr, 1.0, 1);
     else
-        spec_hilbert_leray_kernel<double2><<<spec_rows_grid(g), 128, 0, stream>>>(g, (double2*)f, nullptr, 1.0, 1);
+        launch_k(spec_hilbert_leray_kernel<double2>, spec_rows_grid(g), 128, 0, g, (double2*)f, nullptr, 1.0, 1);
     launched("spec_leray", 6.0 * sv_elem() * g.ncomp, ev);
 }
 
@@ -331,9 +333,9 @@ void EngineBase::hilbert_leray(SVec* f, double order, double scale) {
     const double* t = hilbert_table(order);
     cudaEvent_t ev = prof_mark();
     if (state32_)
-        spec_hilbert_leray_kernel<float2><<<spec_rows_grid(g), 128, 0, stream>>>(g, (float2*)f, t, scale, 1);
+        launch_k(spec_hilbert_leray_kernel<float2>, spec_rows_grid(g), 128, 0, g, (float2*)f, t, scale, 1);
     else
-        spec_hilbert_leray_kernel<double2><<<spec_rows_grid(g), 128, 0, stream>>>(g, (double2*)f, t, scale, 1);
+        launch_k(spec_hilbert_leray_kernel<double2>, spec_rows_grid(g), 128, 0, g, (double2*)f, t, scale, 1);
     launched("spec_hilbert_leray", 6.0 * sv_elem() * g.ncomp, ev);
 }
 
@@ -347,10 +349,10 @@ void EngineBase::hilbert_leray_pair_dots(SVec* f1, SVec* f2, double order, int l
     ensure_partials((long)grid * 2);
     cudaEvent_t ev = prof_mark();
     if (state32_)
-        spec_hilbert_leray_pair_dot_kernel<float2><<<grid, 128, 0, stream>>>(
+        launch_k(spec_hilbert_leray_pair_dot_kernel<float2>, grid, 128, 0, 
             g, (float2*)f1, 1.0, (float2*)f2, d_results + lqq, P.q, t, hw, d_partials);
     else
-        spec_hilbert_leray_pair_dot_kernel<double2><<<grid, 128, 0, stream>>>(
+        launch_k(spec_hilbert_leray_pair_dot_kernel<double2>, grid, 128, 0, 
             g, (double2*)f1, 1.0, (double2*)f2, d_results + lqq, P.q, t, hw, d_partials);
     launched("spec_hilbert_leray", 2 * 6.0 * sv_elem() * g.ncomp, ev);
     finalize(grid, 2, 1.0, RS_CC);
@@ -365,16 +367,16 @@ void EngineBase::direction(SVec* gv, SVec* d, const SVec* td, const SVec* u, boo
     const DirectionArgs a{d_results, normalize ? 1 : 0, conjugate ? 1 : 0, reset ? 1 : 0, g.ncomp};
     cudaEvent_t ev = prof_mark();
     if (state32_)
-        spec_direction_kernel<float2><<<grid_for(nt, 256), 256, 0, stream>>>(nt, (float2*)gv, (float2*)d,
+        launch_k(spec_direction_kernel<float2>, grid_for(nt, 256), 256, 0, nt, (float2*)gv, (float2*)d,
                                                                             (const float2*)td, (const float2*)u, a);
     else
-        spec_direction_kernel<double2><<<grid_for(nt, 256), 256, 0, stream>>>(nt, (double2*)gv, (double2*)d,
+        launch_k(spec_direction_kernel<double2>, grid_for(nt, 256), 256, 0, nt, (double2*)gv, (double2*)d,
                                                                              (const double2*)td, (const double2*)u, a);
     launched("spec_lincomb", (double)sv_elem() * nt * (conjugate && !reset ? 4 : 3), ev);
 }
 
 // ---- spectral inner products ----
-using DotLaunch = void (*)(int, cudaStream_t, const SpecDotArgs&);
+using DotLaunch = void (*)(int, cudaStream_t, bool, const SpecDotArgs&);
 template <class K>
 static int dot_resident(K kernel) {
     int per_sm = 0, dev = 0, sms = 0;
@@ -384,12 +386,12 @@ static int dot_resident(K kernel) {
     return std::max(1, per_sm) * sms;
 }
 template <typename V>
-static void launch_dot_generic(int grid, cudaStream_t s, const SpecDotArgs& a) {
-    spec_dot_kernel<V><<<grid, RED_THREADS, 0, s>>>(a);
+static void launch_dot_generic(int grid, cudaStream_t s, bool pdl, const SpecDotArgs& a) {
+    MLQ_CUDA(launch_pdl(pdl, spec_dot_kernel<V>, grid, RED_THREADS, 0, s, a));
 }
 template <typename V, int NV, int NP, unsigned long long PAT>
-static void launch_dot_fixed(int grid, cudaStream_t s, const SpecDotArgs& a) {
-    spec_dot_fixed_kernel<V, NV, NP, PAT><<<grid, RED_THREADS, 0, s>>>(a);
+static void launch_dot_fixed(int grid, cudaStream_t s, bool pdl, const SpecDotArgs& a) {
+    MLQ_CUDA(launch_pdl(pdl, spec_dot_fixed_kernel<V, NV, NP, PAT>, grid, RED_THREADS, 0, s, a));
 }
 // operand pattern of pair p: vector indices ia, ib
 constexpr unsigned long long dot_pp(int p, int ia, int ib) {
@@ -502,7 +504,7 @@ void EngineBase::dots_async(const SpecDotPair* pairs, int np, SVec* ax_out, cons
     ensure_partials((long)grid * 8);
     a.partials = d_partials;
     cudaEvent_t ev = prof_mark();
-    (fv ? fv->fn[w] : tab.generic[w])(grid, stream, a);
+    (fv ? fv->fn[w] : tab.generic[w])(grid, stream, pdl_, a);
     // vectors read (ax_out only when it is an update operand) and written
     const bool out_read = ax_out && (ax_out == ax_x || ax_out == ax_y);
     const int nread = nv - ((a.ax_last && !out_read) ? 1 : 0);

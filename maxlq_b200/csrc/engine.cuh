@@ -187,6 +187,14 @@ class EngineBase {
     void launched(const char* name = nullptr, double alg_bytes = 0.0, cudaEvent_t a = nullptr);
     cudaEvent_t prof_mark();
     bool prof_on = false;
+    // a launch on the engine's stream that overlaps its predecessor's end
+    // (the kernel calls pdl_begin); off inside the line search's conditional graph
+    // MLQ_PDL=0: plain launches
+    bool pdl_on_ = true, pdl_ = true;
+    template <class... P, class... A>
+    void launch_k(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+        MLQ_CUDA(launch_pdl(pdl_, kernel, grid, block, smem, stream, std::forward<A>(args)...));
+    }
 
     // ---- CUDA graphs of fixed launch sequences ----
     // as_graph(name, key, body): the first call with a key runs body() as is

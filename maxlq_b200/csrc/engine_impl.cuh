@@ -144,7 +144,7 @@ void Engine<T>::xinv_c(XInvArgs<T>& xa, int narr) {
     const int G = persistent_blocks((const void*)kern, S::XTHREADS, smem);
     const long ng = xa.nlines / LPB;
     dim3 grid((unsigned)std::min<long>(ng, std::max(1, G / narr)), narr);
-    kern<<<grid, S::XTHREADS, smem, stream>>>(xa, d_twT_ + tw_off.at(NN / 2), d_twT_ + tw_off.at(NN));
+    this->launch_k(kern, grid, S::XTHREADS, smem, xa, d_twT_ + tw_off.at(NN / 2), d_twT_ + tw_off.at(NN));
 }
 
 // y/z launches of tile-shape variant V (cfft.cuh YShape)
@@ -161,7 +161,7 @@ void Engine<T>::y_cv(YArgs<T>& ya, int sign, int narr) {
                 allow_smem(kern);
                 const int G = persistent_blocks((const void*)kern, PS::THREADS, smem);
                 dim3 grid((unsigned)std::min<long>(items, std::max(1, G / narr)), narr);
-                kern<<<grid, PS::THREADS, smem, stream>>>(ya, d_twT_ + tw_off.at(NN));
+                this->launch_k(kern, grid, PS::THREADS, smem, ya, d_twT_ + tw_off.at(NN));
             };
             if (sign < 0)
                 run(ypass_pair_kernel<NN, -1, S::PAIR_MINB>);
@@ -176,7 +176,7 @@ void Engine<T>::y_cv(YArgs<T>& ya, int sign, int narr) {
         allow_smem(kern);
         const int G = persistent_blocks((const void*)kern, S::YTHREADS, smem);
         dim3 grid((unsigned)std::min<long>(items, std::max(1, G / narr)), narr);
-        kern<<<grid, S::YTHREADS, smem, stream>>>(ya, d_twT_ + tw_off.at(NN));
+        this->launch_k(kern, grid, S::YTHREADS, smem, ya, d_twT_ + tw_off.at(NN));
     };
     if constexpr (S::CW) {
         if (sign < 0)
@@ -206,7 +206,7 @@ void Engine<T>::zfwd_cv(ZFwdArgs<T>& za, int narr) {
             last_zblocks_ = (long)grid.x * narr;
             ensure_partials(last_zblocks_ * MAX_RED);
             za.partials = d_partials;
-            kern<<<grid, PS::THREADS, smem, stream>>>(za, d_twT_ + tw_off.at(NN));
+            this->launch_k(kern, grid, PS::THREADS, smem, za, d_twT_ + tw_off.at(NN));
         }
         return;
     }
@@ -220,7 +220,7 @@ void Engine<T>::zfwd_cv(ZFwdArgs<T>& za, int narr) {
         last_zblocks_ = (long)grid.x * narr;
         ensure_partials(last_zblocks_ * MAX_RED);
         za.partials = d_partials;
-        kern<<<grid, S::YTHREADS, smem, stream>>>(za, d_twT_ + tw_off.at(NN));
+        this->launch_k(kern, grid, S::YTHREADS, smem, za, d_twT_ + tw_off.at(NN));
     };
     if constexpr (S::CW)
         run(zfwd_cw_kernel<NN, V, T>);
@@ -265,7 +265,7 @@ void Engine<T>::zinv_cv(ZInvArgs<T>& za, int narr) {
         allow_smem(kern);
         const int G = persistent_blocks((const void*)kern, S::YTHREADS, smem);
         dim3 grid((unsigned)std::min<long>(items, std::max(1, G / narr)), narr);
-        kern<<<grid, S::YTHREADS, smem, stream>>>(za, d_twT_ + tw_off.at(NN));
+        this->launch_k(kern, grid, S::YTHREADS, smem, za, d_twT_ + tw_off.at(NN));
     };
     if constexpr (S::CW)
         run(zinv_cw_kernel<NN, V, T>);
@@ -542,7 +542,7 @@ void Engine<T>::xfwd_c(XFwdArgs<T>& xa, const F& f) {
     last_xblocks_ = grid;
     if (F::NRED > 0) ensure_partials((long)grid * F::NRED);
     xa.partials = d_partials;
-    kern<<<grid, S::XTHREADS, smem, stream>>>(xa, f, d_twT_ + tw_off.at(NN / 2), d_twT_ + tw_off.at(NN));
+    this->launch_k(kern, grid, S::XTHREADS, smem, xa, f, d_twT_ + tw_off.at(NN / 2), d_twT_ + tw_off.at(NN));
 }
 
 template <typename T>
@@ -742,7 +742,7 @@ void Engine<T>::zinv_multi_cv(ZInvMultiArgs<T>& za, int nops) {
             allow_smem(kern);
             const int G = persistent_blocks((const void*)kern, PS::THREADS, smem);
             dim3 grid((unsigned)std::min<long>(items, std::max(1, G / nops)), nops);
-            kern<<<grid, PS::THREADS, smem, stream>>>(za, d_twT_ + tw_off.at(NN));
+            this->launch_k(kern, grid, PS::THREADS, smem, za, d_twT_ + tw_off.at(NN));
         }
     } else if constexpr (S::CW) {  // the multi-output kernels have the plain and pair tile shapes only
         zinv_multi_cv<NN, 0>(za, nops);
@@ -753,7 +753,7 @@ void Engine<T>::zinv_multi_cv(ZInvMultiArgs<T>& za, int nops) {
         allow_smem(kern);
         const int G = persistent_blocks((const void*)kern, S::YTHREADS, smem);
         dim3 grid((unsigned)std::min<long>(items, std::max(1, G / nops)), nops);
-        kern<<<grid, S::YTHREADS, smem, stream>>>(za, d_twT_ + tw_off.at(NN));
+        this->launch_k(kern, grid, S::YTHREADS, smem, za, d_twT_ + tw_off.at(NN));
     }
 }
 
@@ -1149,7 +1149,7 @@ void Engine<T>::pointwise(const F& f, const std::vector<int>& in, const std::vec
             ensure_partials((long)grid * std::max(F::NRED, 1));
             a.partials = d_partials;
             cudaEvent_t ev = prof_mark();
-            pointwise_kernel<T, F><<<grid, RED_THREADS, 0, stream>>>(a, f);
+            launch_k(pointwise_kernel<T, F>, grid, RED_THREADS, 0, a, f);
             launched("pointwise", (double)a.npts * sizeof(T) * (F::NIN + F::NOUT), ev);
             if (F::NRED > 0 && fred_dst >= 0) finalize(grid, F::NRED, 1.0 / (double)n3, fred_dst, z0 > 0);
         }
@@ -1170,7 +1170,7 @@ void Engine<T>::pointwise(const F& f, const std::vector<int>& in, const std::vec
     ensure_partials((long)grid * std::max(F::NRED, 1));
     a.partials = d_partials;
     cudaEvent_t ev = prof_mark();
-    kern<<<grid, RED_THREADS, 0, stream>>>(a, f);
+    this->launch_k(kern, grid, RED_THREADS, 0, a, f);
     launched("pointwise", (double)n3 * sizeof(T) * (F::NIN + F::NOUT), ev);
     if (F::NRED > 0 && fred_dst >= 0) finalize(grid, F::NRED, 1.0 / (double)n3, fred_dst);
 }
@@ -1327,7 +1327,7 @@ const T* Engine<T>::expand(int i, int z0, int k) {
             const int grid = grid_for(npts, RED_THREADS, 148 * 8);
             a.partials = d_partials;
             cudaEvent_t ev = prof_mark();
-            pointwise_kernel<T, FGPow><<<grid, RED_THREADS, 0, stream>>>(a, fp);
+            launch_k(pointwise_kernel<T, FGPow>, grid, RED_THREADS, 0, a, fp);
             launched("pointwise", (double)npts * sizeof(T) * 2, ev);
             return slab_buf(k);
         }
@@ -1409,6 +1409,7 @@ void Engine<T>::release_io_buffers() {
 template <typename V, typename T>
 __global__ void spec_div_ksq_kernel(SpecGeom g, const V* __restrict__ c0, const V* __restrict__ c1,
                                     const V* __restrict__ c2, cpx<T>* __restrict__ out) {
+    pdl_begin();
     const double twopi = 2.0 * 3.14159265358979311600;
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < g.ncomp; i += (long)gridDim.x * blockDim.x) {
         const int fx = (int)(i % g.nx);
@@ -1669,6 +1670,7 @@ struct SDotArgs {
 
 template <typename T>
 __global__ void __launch_bounds__(RED_THREADS) spec_sdot_kernel(SDotArgs<T> a) {
+    pdl_begin();
     double acc[6] = {0, 0, 0, 0, 0, 0};
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < a.g.ncomp; i += (long)gridDim.x * blockDim.x) {
         const int fx = (int)(i % a.g.nx);
@@ -1695,7 +1697,7 @@ static void sdots(Engine<T>& e, const std::vector<std::pair<const cpx<T>*, const
     e.ensure_partials((long)grid * 6);
     a.partials = e.d_partials;
     cudaEvent_t ev = e.prof_mark();
-    spec_sdot_kernel<T><<<grid, RED_THREADS, 0, e.stream>>>(a);
+    e.launch_k(spec_sdot_kernel<T>, grid, RED_THREADS, 0, a);
     e.launched("spec_sdot", 2.0 * a.np * a.g.ncomp * sizeof(cpx<T>), ev);
     e.finalize(grid, 6, 1.0, dst);
 }
@@ -2022,15 +2024,15 @@ void Engine<T>::grad_l2_body(const SVec* u, SVec* v, SVec* c, bool want_lq, bool
             const int ws2[2] = {WA, WS};
             for (int w : ws2) {
                 cudaEvent_t ew = prof_mark();
-                spec_scale_pow_kernel<cpx<T>><<<grid_for(nsp, 256), 256, 0, stream>>>(wspec(w), wspec(w), nsp, d_coef_, 2);
+                launch_k(spec_scale_pow_kernel<cpx<T>>, grid_for(nsp, 256), 256, 0, wspec(w), wspec(w), nsp, d_coef_, 2);
                 launched("spec_scale", 2.0 * nsp * sizeof(cpx<T>), ew);
             }
             cudaEvent_t ev = prof_mark();
             if (state32_)
-                spec_scale_pow_kernel<float2><<<grid_for(3 * nc, 256), 256, 0, stream>>>(
+                launch_k(spec_scale_pow_kernel<float2>, grid_for(3 * nc, 256), 256, 0, 
                     (float2*)c, (const float2*)c_tmp_, 3 * nc, d_coef_, 3);
             else
-                spec_scale_pow_kernel<double2><<<grid_for(3 * nc, 256), 256, 0, stream>>>(
+                launch_k(spec_scale_pow_kernel<double2>, grid_for(3 * nc, 256), 256, 0, 
                     (double2*)c, (const double2*)c_tmp_, 3 * nc, d_coef_, 3);
             launched("spec_scale", 2.0 * 3 * nc * sv_elem(), ev);
         } else {
@@ -2071,7 +2073,7 @@ void Engine<T>::grad_l2_body(const SVec* u, SVec* v, SVec* c, bool want_lq, bool
             // the line search's coefficient spectra (same symbol)
             const long nsp = (long)b.nb * b.nb * b.nx;
             cudaEvent_t ev = prof_mark();
-            spec_poly3_kernel<cpx<T>><<<grid_for(nsp, 256), 256, 0, stream>>>(
+            launch_k(spec_poly3_kernel<cpx<T>>, grid_for(nsp, 256), 256, 0, 
                 wspec(WP), wspec(WLQ), wspec(WLQ + 1), wspec(WLQ + 2), nsp, 0.0, 0.0, 0.0, d_coef_);
             launched("spec_poly", 4.0 * nsp * sizeof(cpx<T>), ev);
             if (!sac) fwd(b, FSq3{}, {PU, PU + 1, PU + 2}, {oS});
@@ -2145,10 +2147,10 @@ void Engine<T>::grad_l2_body(const SVec* u, SVec* v, SVec* c, bool want_lq, bool
         const SpecGeom g2 = geom(b);
         cudaEvent_t ev = prof_mark();
         if (state32_)
-            spec_div_ksq_kernel<float2, T><<<grid_for(g2.ncomp, 256), 256, 0, stream>>>(
+            launch_k(spec_div_ksq_kernel<float2, T>, grid_for(g2.ncomp, 256), 256, 0, 
                 g2, (const float2*)scomp(c, 0), (const float2*)scomp(c, 1), (const float2*)scomp(c, 2), wspec(WDIV));
         else
-            spec_div_ksq_kernel<double2, T><<<grid_for(g2.ncomp, 256), 256, 0, stream>>>(
+            launch_k(spec_div_ksq_kernel<double2, T>, grid_for(g2.ncomp, 256), 256, 0, 
                 g2, (const double2*)scomp(c, 0), (const double2*)scomp(c, 1), (const double2*)scomp(c, 2),
                 wspec(WDIV));
         launched("spec_scale", (double)g2.ncomp * (3.0 * sv_elem() + sizeof(cpx<T>)), ev);
@@ -2281,7 +2283,7 @@ int Engine<T>::transport_async(const SVec* u, const SVec* d, double tau, const S
         pointwise(f, {ls_phys(0), ls_phys(1), ls_phys(2)}, {PS, PA});
         const long nsp = (long)b2.nb * b2.nb * b2.nx;
         cudaEvent_t ev = prof_mark();
-        spec_poly3_kernel<cpx<T>><<<grid_for(nsp, 256), 256, 0, stream>>>(
+        launch_k(spec_poly3_kernel<cpx<T>>, grid_for(nsp, 256), 256, 0, 
             wspec(WS), wspec(ls_wspec(0)), wspec(ls_wspec(1)), wspec(ls_wspec(2)), nsp, 1.0, tau, tau * tau, nullptr);
         launched("spec_poly", 4.0 * nsp * sizeof(cpx<T>), ev);
         MLQ_CUDA(cudaMemcpyAsync(wspec(WA), wspec(WS), nsp * sizeof(cpx<T>), cudaMemcpyDeviceToDevice, stream));
@@ -2373,6 +2375,7 @@ template <typename T>
 __global__ void __launch_bounds__(RED_THREADS, 4)
     ls_interval_kernel(const T* __restrict__ s0, const T* __restrict__ s1, const T* __restrict__ s2, long npts,
                        LsAnchorSet an, double* __restrict__ out) {
+    pdl_begin();
     constexpr int K = LS_ANCHORS + 1;
     const double inf = 1e300;
     double lo[K], hi[K];
@@ -2440,6 +2443,7 @@ template <typename T>
 __global__ void __launch_bounds__(RED_THREADS)
     ls_min_kernel(const T* __restrict__ s0, const T* __restrict__ s1, const T* __restrict__ s2, long npts, double tau,
                   const double* __restrict__ taup, double* __restrict__ out) {
+    pdl_begin();
     const T t = (T)(taup ? *taup : tau);
     T m = T(1e30);
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < npts; i += (long)gridDim.x * blockDim.x)
@@ -2582,7 +2586,7 @@ void Engine<T>::ls_interval_dev(double tau0) {
     const int grid = grid_for(n3, RED_THREADS, 148 * 4);
     ensure_partials((long)grid * 2 * (LS_ANCHORS + 1));
     cudaEvent_t ev = prof_mark();
-    ls_interval_kernel<T><<<grid, RED_THREADS, 0, stream>>>(phys(ls_phys(0)), phys(ls_phys(1)), phys(ls_phys(2)), n3,
+    launch_k(ls_interval_kernel<T>, grid, RED_THREADS, 0, phys(ls_phys(0)), phys(ls_phys(1)), phys(ls_phys(2)), n3,
                                                             an, d_partials);
     launched("ls_interval", 3.0 * n3 * sizeof(T), ev);
     ls_launch_coef(d_ls_, d_results, d_partials, grid, an, stream);
@@ -2602,6 +2606,7 @@ struct LsDotArgs {
 };
 template <typename T>
 __global__ void __launch_bounds__(RED_THREADS) spec_ls_dot_kernel(LsDotArgs<T> a) {
+    pdl_begin();
     double acc[15];
 #pragma unroll
     for (int r = 0; r < 15; ++r) acc[r] = 0.0;
@@ -2659,7 +2664,7 @@ void Engine<T>::ls_setup(const SVec* u, const SVec* d, double tau0) {
         ensure_partials((long)grid * 15);
         a.partials = d_partials;
         cudaEvent_t ev = prof_mark();
-        spec_ls_dot_kernel<T><<<grid, RED_THREADS, 0, stream>>>(a);
+        launch_k(spec_ls_dot_kernel<T>, grid, RED_THREADS, 0, a);
         launched("spec_sdot", 6.0 * a.g.ncomp * sizeof(cpx<T>), ev);
         finalize(grid, 15, 1.0, 140);
     }
@@ -2689,7 +2694,7 @@ void Engine<T>::ls_setup(const SVec* u, const SVec* d, double tau0) {
             } else {
                 for (int a = 0; a < 3; ++a) s[a] = phys(ls_phys(a));
             }
-            ls_interval_kernel<T><<<grid, RED_THREADS, 0, stream>>>(s[0], s[1], s[2], npts, an, d_partials);
+            launch_k(ls_interval_kernel<T>, grid, RED_THREADS, 0, s[0], s[1], s[2], npts, an, d_partials);
             launched();
             MLQ_CUDA(cudaMemcpyAsync(h.data(), d_partials, h.size() * sizeof(double), cudaMemcpyDeviceToHost, stream));
             MLQ_CUDA(cudaStreamSynchronize(stream));
@@ -2769,6 +2774,7 @@ bool Engine<T>::ls_graph_build(LsGraph& g, int key) {
     const std::vector<int> in = {ls_phys(0), ls_phys(1), ls_phys(2)};
     const bool prof_was = prof_on;
     prof_on = false;
+    pdl_ = false;  // the conditional bodies keep full dependencies
     // one transform trial run directly, so that the buffers it allocates on
     // first use exist before the capture (its sums land in unused slots)
     FLSA f0;
@@ -2806,7 +2812,7 @@ bool Engine<T>::ls_graph_build(LsGraph& g, int key) {
             cudaGraph_t body_chk = add_conditional(body_loop, graph_leaf(body_loop), h_chk, cudaGraphCondTypeIf);
             MLQ_CUDA(cudaGraphConditionalHandleCreate(&h_fft, body_chk, 0, cudaGraphCondAssignDefault));
             capture_into(body_chk, [&] {
-                ls_min_kernel<T><<<grid, RED_THREADS, 0, stream>>>(phys(in[0]), phys(in[1]), phys(in[2]), n3, 0.0,
+                launch_k(ls_min_kernel<T>, grid, RED_THREADS, 0, phys(in[0]), phys(in[1]), phys(in[2]), n3, 0.0,
                                                                    &d_ls_->ptau, d_partials);
                 ls_launch_check(d_ls_, d_partials, grid, h_fft, stream);
             });
@@ -2826,6 +2832,7 @@ bool Engine<T>::ls_graph_build(LsGraph& g, int key) {
     cudaGetLastError();
     launches = l0 + nfwd;  // captured launches did not run
     prof_on = prof_was;
+    pdl_ = pdl_on_;
     if (!ok) {
         if (exec) cudaGraphExecDestroy(exec);
         return false;
@@ -2906,7 +2913,7 @@ bool Engine<T>::ls_clamp_free(double tau) {
                 for (int a = 0; a < 3; ++a) sp[a] = phys(ls_phys(a));
             }
             cudaEvent_t ev = prof_mark();
-            ls_min_kernel<T><<<grid, RED_THREADS, 0, stream>>>(sp[0], sp[1], sp[2], npts, tau, nullptr, d_partials);
+            launch_k(ls_min_kernel<T>, grid, RED_THREADS, 0, sp[0], sp[1], sp[2], npts, tau, nullptr, d_partials);
             launched("ls_min", 3.0 * npts * sizeof(T), ev);
             MLQ_CUDA(cudaMemcpyAsync(h.data(), d_partials, h.size() * sizeof(double), cudaMemcpyDeviceToHost, stream));
             MLQ_CUDA(cudaStreamSynchronize(stream));
@@ -3013,6 +3020,7 @@ struct PolyDotArgs {
 };
 template <typename T, int NA, int NB, bool SAME>
 __global__ void __launch_bounds__(RED_THREADS) spec_polydot_kernel(PolyDotArgs<T, NA, NB> a) {
+    pdl_begin();
     constexpr int NR = NA + NB - 1;
     double acc[NR];
 #pragma unroll
@@ -3042,7 +3050,7 @@ static void polydot(Engine<T>& e, int wa, int wb, int dst) {
     e.ensure_partials((long)grid * (NA + NB - 1));
     a.partials = e.d_partials;
     cudaEvent_t ev = e.prof_mark();
-    spec_polydot_kernel<T, NA, NB, SAME><<<grid, RED_THREADS, 0, e.stream>>>(a);
+    e.launch_k(spec_polydot_kernel<T, NA, NB, SAME>, grid, RED_THREADS, 0, a);
     e.launched("spec_sdot", (double)(SAME ? NA : NA + NB) * a.g.ncomp * sizeof(cpx<T>), ev);
     e.finalize(grid, NA + NB - 1, 1.0, dst);
 }
@@ -3193,7 +3201,7 @@ void Engine<T>::lsg_trial(double tau, double out[3], double* lqq) {
         pointwise(f, s3, {LTS, LTA});
         const long nsp = (long)b2.nb * b2.nb * b2.nx;
         cudaEvent_t ev = prof_mark();
-        spec_poly3_kernel<cpx<T>><<<grid_for(nsp, 256), 256, 0, stream>>>(
+        launch_k(spec_poly3_kernel<cpx<T>>, grid_for(nsp, 256), 256, 0, 
             wspec(WA), wspec(ls_wspec(0)), wspec(ls_wspec(1)), wspec(ls_wspec(2)), nsp, 1.0, tau, tau * tau, nullptr);
         launched("spec_poly", 4.0 * nsp * sizeof(cpx<T>), ev);
     } else {

@@ -56,6 +56,7 @@ static __global__ void __launch_bounds__(FIN_THREADS)
                              double* __restrict__ results, int dst, int accumulate) {
     __shared__ double sm[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    pdl_begin<true>();
     const int per = nr < nw ? nw / nr : 1;  // warps per sum
     for (int r0 = 0; r0 < nr; r0 += nw) {
         const int r = r0 + warp / per, w = warp % per;
@@ -173,6 +174,7 @@ template <typename T, class F>
 __global__ void __launch_bounds__(RED_THREADS) pointwise_kernel(PArgs<T> a, F f) {
     constexpr int NIN = F::NIN, NOUT = F::NOUT, NR = F::NRED;
     using T2 = cpx<T>;  // two consecutive points per load and store
+    pdl_begin();
     double acc[NR > 0 ? NR : 1];
 #pragma unroll
     for (int r = 0; r < (NR > 0 ? NR : 1); ++r) acc[r] = 0.0;
@@ -669,6 +671,7 @@ __device__ __forceinline__ void spec_coords(const SpecGeom& g, long i, int& fx, 
 template <typename V>
 __global__ void spec_lincomb_kernel(SpecGeom g, V* out, double a, const V* x, double b, const V* y, double c,
                                     const V* z) {
+    pdl_begin();
     const long nt = 3 * g.ncomp;
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < nt; i += (long)gridDim.x * blockDim.x) {
         double2 v = ldv(x, i);
@@ -691,6 +694,7 @@ __global__ void spec_lincomb_kernel(SpecGeom g, V* out, double a, const V* x, do
 // the factor read from device memory (stays valid in a replayed graph)
 template <typename C>
 __global__ void spec_scale_pow_kernel(C* out, const C* in, long n, const double* coef, int pw) {
+    pdl_begin();
     double f = 1.0;
     for (int k = 0; k < pw; ++k) f *= coef[0];
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
@@ -706,6 +710,7 @@ __global__ void spec_scale_pow_kernel(C* out, const C* in, long n, const double*
 template <typename C>
 __global__ void spec_poly3_kernel(C* out, const C* a, const C* b, const C* c, long n, double c0, double c1,
                                   double c2, const double* coef) {
+    pdl_begin();
     if (coef) {
         c0 = coef[0] * coef[0];
         c1 = c0 * coef[1];
@@ -731,6 +736,7 @@ struct TransportArgs {
 };
 template <typename V>
 __global__ void spec_transport_kernel(long nt, const V* g, const V* d, V* u, V* tg, V* td, TransportArgs a) {
+    pdl_begin();
     __shared__ double f[3];
     if (threadIdx.x == 0) {
         const double ln = pow(a.results[a.lnq_slot], 1.0 / a.q), cs = a.B / ln, fq = pow(ln, -a.q);
@@ -795,6 +801,7 @@ __device__ __forceinline__ void hilbert_leray_point(double2& u0, double2& u1, do
 template <typename V>
 __global__ void spec_hilbert_leray_kernel(SpecGeom g, V* f, const double* __restrict__ htab, double scale,
                                           int do_leray) {
+    pdl_begin();
     const double twopi = 2.0 * 3.14159265358979311600;
     const int nrows = g.nb * g.nb;
     // one warp per row (kx across the lanes), blockDim / 32 rows per block pass
@@ -829,6 +836,7 @@ __global__ void __launch_bounds__(128) spec_hilbert_leray_pair_dot_kernel(SpecGe
                                                                        const double* __restrict__ htab,
                                                                        const double* __restrict__ hwtab,
                                                                        double* partials) {
+    pdl_begin();
     __shared__ double s2sh;  // ||u||_q^{1-q} from ||u||_q^q
     if (threadIdx.x == 0) s2sh = pow(pow(*lqq, 1.0 / q), 1.0 - q);
     __syncthreads();
@@ -879,6 +887,7 @@ struct DirectionArgs {
 };
 template <typename V>
 __global__ void spec_direction_kernel(long nt, V* g, V* d, const V* td, const V* u, DirectionArgs a) {
+    pdl_begin();
     double sg, beta;
     cg_direction_factors(a.results + RS_IP, a.normalize, a.conjugate, a.reset, sg, beta);
     const long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -974,6 +983,7 @@ __device__ __forceinline__ double dot_ax_factor(const SpecDotArgs& a) {
 // pattern of operands).  One warp per row, each lane one mode at a time.
 template <typename V>
 __global__ void __launch_bounds__(RED_THREADS) spec_dot_kernel(SpecDotArgs a) {
+    pdl_begin();
     double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     const SpecGeom& g = a.g;
     const double ax_a = dot_ax_factor(a);
@@ -1023,6 +1033,7 @@ __global__ void __launch_bounds__(RED_THREADS) spec_dot_kernel(SpecDotArgs a) {
 // replaces vec[NV - 1] when ax_last).
 template <typename V, int NV, int NP, unsigned long long PAT>
 __global__ void __launch_bounds__(RED_THREADS) spec_dot_fixed_kernel(SpecDotArgs a) {
+    pdl_begin();
     double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     const SpecGeom& g = a.g;
     const double ax_a = dot_ax_factor(a);

@@ -89,6 +89,7 @@ constexpr int LS_COEF_THREADS = 512;
 __global__ void __launch_bounds__(LS_COEF_THREADS)
     ls_coef_kernel(LsDevState* s, const double* __restrict__ results, const double* __restrict__ partials, int nblocks,
                    LsAnchorSet an) {
+    pdl_begin();
     // max and min are exact, so any order gives the same ends; one warp alone
     // took 20 us over the 592 blocks of 64^3
     constexpr int K = LS_ANCHORS + 1, W = 2 * K, NW = LS_COEF_THREADS / 32;
@@ -231,7 +232,7 @@ __global__ void ls_fft_kernel(LsDevState* s, const double* __restrict__ r) {
 
 void ls_launch_coef(LsDevState* s, const double* results, const double* partials, int nblocks, const LsAnchorSet& an,
                     cudaStream_t st) {
-    ls_coef_kernel<<<1, LS_COEF_THREADS, 0, st>>>(s, results, partials, nblocks, an);
+    MLQ_CUDA(launch_pdl(true, ls_coef_kernel, 1, LS_COEF_THREADS, 0, st, s, results, partials, nblocks, an));
 }
 void ls_launch_ctrl(LsDevState* s, cudaGraphConditionalHandle h_loop, cudaGraphConditionalHandle h_chk,
                     cudaStream_t st) {
