@@ -321,8 +321,9 @@ struct CShape {
                                                : (L >= 512 ? 16 : (L >= 64 ? 8 : 4));
     static constexpr int TPLX = L / EX;
     // threads per x block: 12 FP64 elements per thread would park more than
-    // an SM's shared memory in a six-output forward block of 256
-    static constexpr int XTHREADS = THREE && EX == 12 && sizeof(T) == 8 ? 128 : 256;
+    // an SM's shared memory in a six-output forward block of 256; 8 take three
+    // blocks of 128 (xfwd_minb)
+    static constexpr int XTHREADS = sizeof(T) == 8 && EX >= 8 ? 128 : 256;
     // x pass twiddles: registers in FP32; a shared-memory table in FP64,
     // where the registers are needed for the data
     static constexpr bool XTW_REG = sizeof(T) == 4;
@@ -541,14 +542,18 @@ __host__ __device__ constexpr int xfwd_chunk(int nin, int e) {
     return c;
 }
 
-// resident blocks the register budget aims at: light functors 2, heavy ones 1
-template <class F>
+// Resident blocks the register budget aims at: light functors 512 threads per
+// SM, heavy ones 256.  FP64 with 8 elements and up to 3 outputs: 384 in blocks
+// of 128 (170 registers), which the loads of a heavy functor need to hide the
+// transforms of its outputs: FG3 at 256^3 0.83 -> 0.69 ms; four outputs and
+// more lose by it (FLSTrialE at 128^3 82 -> 107 us), as 12 elements do.
+template <class F, typename T, int E, int THREADS>
 constexpr int xfwd_minb() {
-    return F::NIN + F::NOUT <= 8 ? 2 : 1;
+    return F::NIN + F::NOUT <= 8 ? 512 / THREADS : (sizeof(T) == 8 && E == 8 && F::NOUT <= 3 ? 384 : 256) / THREADS;
 }
 
 template <int N, typename T, class F>
-__global__ void __launch_bounds__(CShape<N, T>::XTHREADS, xfwd_minb<F>() * 256 / CShape<N, T>::XTHREADS)
+__global__ void __launch_bounds__(CShape<N, T>::XTHREADS, xfwd_minb<F, T, CShape<N, T>::EX, CShape<N, T>::XTHREADS>())
     xfwd_c_kernel(XFwdArgs<T> a, F f, const cpx<T>* __restrict__ twL, const cpx<T>* __restrict__ twN) {
     using S = CShape<N, T>;
     constexpr int NIN = F::NIN, NOUT = F::NOUT, NR = F::NRED;
