@@ -458,7 +458,10 @@ class Engine : public EngineBase {
     bool lsg_fit_ = false;
     void lsg_setup(const SVec* u, const SVec* d, double tau0 = 0.0);
     void lsg_trial(double tau, double out[3], double* lqq);
-    int lsg_power_sq(double k);
+    // ||.||^2 of the power |.|^k of the S and A that the chain reads
+    int power_sq(double k);
+    // some power of R, the gradient or the norm is a product with A = P2(g^2)
+    bool need_A() const { return P.q + MACH_EPSILON >= 4.0; }
     // even q (6 and 8): the coefficients of the trial's integrals where S(tau)
     // >= 0 at every point (at q = 6 the norm takes one transform per trial)
     bool lsg_poly_ok() const { return !use_e_u && (P.q == 6.0 || P.q == 8.0); }
@@ -620,9 +623,7 @@ class Engine : public EngineBase {
         spec_next_ = 0;
     }
     PowField chain(double k);
-    void ensure_p2_spec(PowField& f);
     void ensure_phys(PowField& f);
-    cpx<T>* ones_spec();
     void A_and_S(bool need_A_phys);
     int lx_for(int nout, size_t extra = 0) const;
     int tx_for() const;

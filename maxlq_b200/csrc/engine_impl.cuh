@@ -1447,7 +1447,7 @@ enum : int {
     PIO3 = 42,  // second host transfer buffer
 };
 // work spectra (band b2)
-enum : int { WG2 = 0, WA = 1, WP = 2, WT = 3 /*3..5*/, WONE = 6, WCH = 7 /*7..*/ };
+enum : int { WG2 = 0, WA = 1, WP = 2, WT = 3 /*3..5*/, WCH = 7 /*7..*/ };
 enum : int { WDIV = 52 };  // -i (K . c) / |K|^2 of the gradient program
 }  // namespace
 // line search along phi = u + tau d (q = 4): physical fields and work spectra
@@ -1476,6 +1476,8 @@ enum : int {
     LE = 124,   // 124..126
     LC = 127,   // 127..131 coefficients of |phi|^{q-4} at q = 8
     LEND = 132,
+    PG2 = 133,  // P2(|grad u|^2) of R
+    WRS = 51,   // work spectrum of S of R
     WTA2 = 54,  // work spectrum of |phi|^{q-2} (e_u branch)
     WLC = 55,   // 55..59 spectra of C
     WLP = 60,   // 60..66 coefficients of P2(p C)
@@ -1529,21 +1531,6 @@ static constexpr int wf64() {
     return sizeof(T) == 8 ? 1 : 0;
 }
 
-// Fourier coefficients of the constant 1 in band b2: a unit k=0 mode.
-template <typename T>
-cpx<T>* Engine<T>::ones_spec() {
-    static_assert(sizeof(cpx<T>) == 2 * sizeof(T), "layout");
-    const bool fresh = (int)ws_.size() <= WONE || ws_[WONE] == nullptr;
-    cpx<T>* w = wspec(WONE);
-    if (fresh) {
-        MLQ_CUDA(cudaMemsetAsync(w, 0, spec_ncomp() * sizeof(cpx<T>), stream));
-        const cpx<T> one = mk<T>(T(1), T(0));
-        MLQ_CUDA(cudaMemcpyAsync(w, &one, sizeof(cpx<T>), cudaMemcpyHostToDevice, stream));
-        MLQ_CUDA(cudaStreamSynchronize(stream));
-    }
-    return w;
-}
-
 template <typename T>
 void Engine<T>::ensure_phys(PowField& f) {
     if (f.phys >= 0) return;
@@ -1561,22 +1548,6 @@ void Engine<T>::ensure_phys(PowField& f) {
         return;
     }
     throw CudaError("power field without physical values", MLQ_ERR_CUDA);
-}
-
-// make sure a power field has a spectrum in band b2
-template <typename T>
-void Engine<T>::ensure_p2_spec(PowField& f) {
-    if (f.spec >= 0) return;
-    if (f.kind == PowField::ONE) {
-        ones_spec();
-        f.spec = WONE;
-        return;
-    }
-    f.spec = WCH + 16 + spec_next_++;
-    FwdOut o;
-    o.spec = wspec(f.spec);
-    o.spec_f64 = wf64<T>();
-    fwd(b2, FCopy{}, {f.phys}, {o});
 }
 
 // S = P2(|u|^2) (calc_uk 2332-2333) must already be in phys(PS) ; computes
@@ -1706,12 +1677,14 @@ static void sdots(Engine<T>& e, const std::vector<std::pair<const cpx<T>*, const
 // together with ||phi||_q^q (calc_global_Lq_norm 1675-1692).  Products are
 // dealiased as the reference does; a dealias that is immediately followed by
 // an L2 inner product with a band-limited field is applied through Parseval
-// on the band instead of by a round trip (the projection is self-adjoint).
+// on the band instead of by a round trip, or not at all where that field is in
+// physical space (the projection is self-adjoint).  At q = 6: 7 forward and 19
+// inverse transforms (12 and 20 with every product transformed): 14.9 -> 12.5 ms
+// at 512^3 mixed, 3.66 -> 2.97 at 256^3 FP64; at q = 4 2.79 -> 2.46.
 template <typename T>
 void Engine<T>::R_eval(const SVec* u, const SVec* d, double tau, double out[3], double* lqq) {
     pu_of_ = nullptr;
     const Band& b = b2;
-    const long nc = spec_ncomp();
     const double q = P.q, cv = P.visc_coef * P.visc, cp = P.press_coef;
     chain_reset();
     // 1. phi and grad phi
@@ -1731,103 +1704,104 @@ void Engine<T>::R_eval(const SVec* u, const SVec* d, double tau, double out[3], 
     for (int i = 0; i < 3; ++i) uin.push_back(PU + i);
     for (int i = 0; i < 9; ++i) uin.push_back(PD + i);
     // 2. first products: |u|^2 -> P2, W_j -> P2 (q>=4), grad u:grad u^T -> p,
-    //    |grad u|^2 -> spectrum
+    //    |grad u|^2
+    const bool direct_q4 = !use_e_u && q == 4.0;  // |u|^{q-4} = 1
     FwdOut oS, oQ, oG2;
     oS.phys_out = PS;
     oQ.sym = SYM_INV_KSQ;  // p = -Lap^-1 P2(grad u : grad u^T) (1339-1340)
     oQ.phys_out = PP;
-    oG2.spec = wspec(WG2);
-    oG2.spec_f64 = wf64<T>();
-    if (!use_e_u) {
+    if (direct_q4) {
+        oG2.spec = wspec(WG2);
+        oG2.spec_f64 = wf64<T>();
+    } else {
+        oG2.phys_out = PG2;
+    }
+    if (use_e_u) {
+        fwd(b, FRProdE{}, uin, {oS, oQ, oG2});
+    } else if (reuse_on_ && 3 * b2.cut < n) {
+        // P2(W_j) = (1/2) d_j S (ls_w_fields): three inverse transforms from
+        // one spectrum instead of three round trips
+        oS.spec = wspec(WRS);
+        oS.spec_f64 = wf64<T>();
+        fwd(b, FRProdE{}, uin, {oS, oQ, oG2});
+        std::vector<InvOut> g;
+        for (int j = 0; j < 3; ++j) {
+            InvOut o;
+            o.nsrc = 1;
+            o.src[0] = ZSrc{wspec(WRS), wf64<T>(), SYM_IKX + j, 0, 0.5};
+            o.phys_out = PV + j;
+            g.push_back(o);
+        }
+        inv(b, g);
+    } else {
         FwdOut oW[3];
         for (int j = 0; j < 3; ++j) oW[j].phys_out = PV + j;
         fwd(b, FRProd{}, uin, {oS, oW[0], oW[1], oW[2], oQ, oG2});
-    } else {
-        fwd(b, FRProdE{}, uin, {oS, oQ, oG2});
     }
-    // 3. |u|^k fields
-    const bool needA = !(q == 4.0 && !use_e_u);  // for q = 4 only the spectrum of A is read
-    A_and_S(needA);
-    PowField a2 = chain(q - 2.0);
-    PowField a4;
-    if (!use_e_u) a4 = chain(q - 4.0);
-    PowField ah = chain(q / 2.0);
+    // 3. |u|^k fields and their products
+    if (need_A()) A_and_S(!direct_q4);  // for q = 4 only the spectrum of A is read
     std::vector<std::pair<const cpx<T>*, const cpx<T>*>> pr;
-    // R1 = -vc nu <a2, P2|grad u|^2>  (1318)
-    ensure_p2_spec(a2);
-    pr.push_back({wspec(a2.spec), wspec(WG2)});
-    // ||phi||_q^q = int (|u|^{q/2})^2
-    bool norm_raw = false;
-    if (ah.kind == PowField::RAW) {
-        norm_raw = true;
-        pointwise(FSqRed{}, {ah.phys}, {}, 20);
-    } else if (ah.spec < 0) {
-        // a band-limited power in a wider band than P2: its full spectrum is
-        // needed; integrate its square in physical space instead
-        norm_raw = true;
-        pointwise(FSqRed{}, {ah.phys}, {}, 20);
-    } else {
-        if (ah.kind == PowField::ONE) ensure_p2_spec(ah);
-        pr.push_back({wspec(ah.spec), wspec(ah.spec)});
+    FwdOut o[4];
+    const int ws[4] = {WT, WT + 1, WT + 2, WTA2};
+    for (int i = 0; i < 4; ++i) {
+        o[i].spec = wspec(ws[i]);
+        o[i].spec_f64 = wf64<T>();
     }
-    const bool direct = !use_e_u && a4.kind == PowField::ONE;
-    if (direct) {
-        // |u|^{q-4} = 1: R2 = -(q-2) vc nu int sum V^2, R3 = (q-2) pc int p u.V
-        pointwise(FRRed1{}, {PV, PV + 1, PV + 2, PP, PU, PU + 1, PU + 2},
-                  {}, 16);
+    const bool raw_a4 = q - 4.0 + MACH_EPSILON < 2.0;  // |u|^{q-4} is outside the band (q branch)
+    if (direct_q4) {
+        // R1 = -vc nu <A, P2|grad u|^2> (1318), R2 = -(q-2) vc nu int sum V^2,
+        // R3 = (q-2) pc int p u.V, ||phi||_4^4 = <A, A>
+        pointwise(FRRed1{}, {PV, PV + 1, PV + 2, PP, PU, PU + 1, PU + 2}, {}, 16);
+        pr = {{wspec(WA), wspec(WG2)}, {wspec(WA), wspec(WA)}};
     } else if (!use_e_u) {
+        PowField a4 = chain(q - 4.0);
         ensure_phys(a4);
-        ensure_p2_spec(a4);
-        FwdOut o[3];
-        for (int i = 0; i < 3; ++i) {
-            o[i].spec = wspec(WT + i);
-            o[i].spec_f64 = wf64<T>();
+        const bool direct = q - 2.0 + MACH_EPSILON < 2.0;
+        int a = PA;
+        if (direct) {
+            PowField a2 = chain(q - 2.0);
+            ensure_phys(a2);
+            a = a2.phys;
         }
-        fwd(b, FRProd2{},
-            {PV, PV + 1, PV + 2, PP, PU, PU + 1, PU + 2, a4.phys},
-            {o[0], o[1], o[2]});
-        pr.push_back({wspec(a4.spec), wspec(WT)});
-        pr.push_back({wspec(WT + 1), wspec(WT + 2)});
+        const std::vector<int> in = {PV, PV + 1, PV + 2, PP, PU, PU + 1, PU + 2, a4.phys, a, PG2};
+        pr = {{wspec(WT + 1), wspec(WT + 2)}};
+        if (raw_a4) {
+            FRTrial<true> f;
+            f.direct = direct;
+            fwd(b, f, in, {o[1], o[2], o[0], o[3]}, -1, 16);
+            pr.push_back({wspec(WT), wspec(WTA2)});
+        } else {
+            FRTrial<false> f;
+            f.direct = direct;
+            fwd(b, f, in, {o[1], o[2]}, -1, 16);
+        }
     } else {
         // E_j = P2(sum_i e_i d_j u_i) (calc_vgraduvgradu / calc_vvgradu, v = e_u)
+        PowField a2 = chain(q - 2.0);
+        ensure_phys(a2);
         std::vector<int> ein = uin;
         ein.push_back(PS);
         FwdOut oE[3];
         for (int j = 0; j < 3; ++j) oE[j].phys_out = PV + j;
         fwd(b, FRE{}, ein, {oE[0], oE[1], oE[2]});
-        ensure_phys(a2);
-        FwdOut o[3];
-        for (int i = 0; i < 3; ++i) {
-            o[i].spec = wspec(WT + i);
-            o[i].spec_f64 = wf64<T>();
-        }
-        fwd(b, FRProd2E{},
-            {PV, PV + 1, PV + 2, PP, PU, PU + 1, PU + 2, PS,
-             a2.phys},
-            {o[0], o[1], o[2]});
-        pr.push_back({wspec(a2.spec), wspec(WT)});
-        pr.push_back({wspec(WT + 1), wspec(WT + 2)});
+        fwd(b, FRTrialE{}, {PV, PV + 1, PV + 2, PP, PU, PU + 1, PU + 2, PS, a2.phys, PG2}, {o[0], o[1], o[2], o[3]},
+            -1, 16);
+        pr = {{wspec(WT + 1), wspec(WT + 2)}, {wspec(WT), wspec(WTA2)}};
     }
+    const int slot = direct_q4 ? 1 : power_sq(q / 2.0);  // ||phi||_q^q = int (|u|^{q/2})^2
     sdots(*this, pr, 0);
     fetch_results();
-    int idx = 0;
-    const double I1 = h_results[idx++];
-    const double nrm = norm_raw ? h_results[20] : h_results[idx++];
-    double I2, I3;
-    if (direct) {
-        I2 = h_results[16];
-        I3 = h_results[17];
-    } else {
-        I2 = h_results[idx++];
-        I3 = h_results[idx++];
-    }
+    const double* r = h_results;
+    const double I1 = direct_q4 ? r[0] : r[16];
+    const double I2 = direct_q4 ? r[16] : (use_e_u || raw_a4 ? r[1] : r[17]);
+    const double I3 = direct_q4 ? r[17] : r[0];
     const double R1 = -cv * I1;
     const double R2 = -cv * (q - 2.0) * I2;
     const double R3 = cp * (q - 2.0) * I3;
     out[0] = R1 + R2 + R3;
     out[1] = R1 + R2;
     out[2] = R3;
-    if (lqq) *lqq = nrm;
+    if (lqq) *lqq = r[slot];
 }
 
 // ----------------------------------------------------------------------------
@@ -2094,11 +2068,10 @@ void Engine<T>::grad_l2_body(const SVec* u, SVec* v, SVec* c, bool want_lq, bool
         inv(b, g);
     }
     // 4. |u|^k fields
-    if (!sac) A_and_S(true);
+    if (!sac && need_A()) A_and_S(true);
     PowField a2 = chain(q - 2.0);
     PowField a4;
     if (!use_e_u) a4 = chain(q - 4.0);
-    PowField ah = chain(q / 2.0);
     ensure_phys(a2);
     // 5. aux2 and c = P2(a2 u) (1115-1153)
     {
@@ -2198,16 +2171,7 @@ void Engine<T>::grad_l2_body(const SVec* u, SVec* v, SVec* c, bool want_lq, bool
             fwd(b, f, in3, {o[0], o[1], o[2]});
         }
     }
-    if (want_lq) {
-        if (ah.kind == PowField::RAW || ah.spec < 0) {
-            pointwise(FSqRed{}, {ah.phys}, {}, 20);
-            grad_lq_slot_ = 20;
-        } else {
-            ensure_p2_spec(ah);
-            sdots(*this, {{wspec(ah.spec), wspec(ah.spec)}}, 0);
-            grad_lq_slot_ = 0;
-        }
-    }
+    if (want_lq) grad_lq_slot_ = power_sq(q / 2.0);
 }
 
 // ||u + tau d||_q^q (calc_global_Lq_norm)
@@ -2231,17 +2195,10 @@ double Engine<T>::lq_pow(const SVec* u, const SVec* d, double tau) {
     FwdOut oS;
     oS.phys_out = PS;
     fwd(b2, FSq3{}, {PU, PU + 1, PU + 2}, {oS});
-    A_and_S(true);
-    PowField ah = chain(P.q / 2.0);
-    if (ah.kind == PowField::RAW || ah.spec < 0) {
-        pointwise(FSqRed{}, {ah.phys}, {}, 20);
-        fetch_results();
-        return h_results[20];
-    }
-    ensure_p2_spec(ah);
-    sdots(*this, {{wspec(ah.spec), wspec(ah.spec)}}, 0);
+    if (need_A()) A_and_S(true);
+    const int slot = power_sq(P.q / 2.0);
     fetch_results();
-    return h_results[0];
+    return h_results[slot];
 }
 
 // vectorTransport (function_ops.f90:1716-1768) pieces at w = u + tau d.
@@ -2293,10 +2250,9 @@ int Engine<T>::transport_async(const SVec* u, const SVec* d, double tau, const S
         oS.spec = wspec(WS);
         oS.spec_f64 = wf64<T>();
         fwd(b2, FSq3{}, {PU, PU + 1, PU + 2}, {oS});
-        A_and_S(true);
+        if (need_A()) A_and_S(true);
     }
     PowField a2 = chain(q - 2.0);
-    PowField ah = chain(q / 2.0);
     if (!c_tmp_) c_tmp_ = alloc_state();
     SVec* cbuf = c_tmp_;
     if (q - 2.0 > MACH_EPSILON) {
@@ -2317,14 +2273,7 @@ int Engine<T>::transport_async(const SVec* u, const SVec* d, double tau, const S
         if (a2.kind != PowField::ONE) throw CudaError("vectorTransport with 2 < q < 2+eps", MLQ_ERR_BADARG);
         lincomb(cbuf, 1.0, u, d ? tau : 0.0, d, 0.0, nullptr);
     }
-    int slot = 0;
-    if (ah.kind == PowField::RAW || ah.spec < 0) {
-        slot = 20;
-        pointwise(FSqRed{}, {ah.phys}, {}, slot);
-    } else {
-        ensure_p2_spec(ah);
-        sdots(*this, {{wspec(ah.spec), wspec(ah.spec)}}, slot);
-    }
+    const int slot = power_sq(q / 2.0);
     SpecDotPair pr[6];
     for (int i = 0; i < nxi; ++i) pr[i] = SpecDotPair{cbuf, xi[i], 0};
     dots_async(pr, nxi);
@@ -3111,7 +3060,7 @@ void Engine<T>::lsg_poly_setup() {
 // chain is only summed (Parseval in the band that dealiases it), so it needs
 // no inverse transform.  Returns the result slot.
 template <typename T>
-int Engine<T>::lsg_power_sq(double k) {
+int Engine<T>::power_sq(double k) {
     FwdOut o;
     o.red_self = 0;
     constexpr int DST = 130;
@@ -3140,6 +3089,10 @@ int Engine<T>::lsg_power_sq(double k) {
         }
     }
     PowField f = chain(k);
+    if (f.spec >= 0) {  // in the band: its spectrum
+        sdots(*this, {{wspec(f.spec), wspec(f.spec)}}, 24);
+        return 24;
+    }
     ensure_phys(f);
     pointwise(FSqRed{}, {f.phys}, {}, 20);
     return 20;
@@ -3272,7 +3225,7 @@ void Engine<T>::lsg_trial(double tau, double out[3], double* lqq) {
             fwd(b2, f, in, {o[1], o[2]}, -1, 16);
         }
     }
-    const int slot = lsg_power_sq(q / 2.0);
+    const int slot = power_sq(q / 2.0);
     sdots(*this, pr, 0);
     fetch_results();
     result(h_results[16], use_e_u || raw_a4 ? h_results[1] : h_results[17], h_results[0]);

@@ -9,7 +9,7 @@
 #define MLQ_XFWD_FUNCTORS(X, P, T, N)                                                                             \
     X(P, T, N, FCopy) X(P, T, N, FMul) X(P, T, N, FSq3) X(P, T, N, FGSq) X(P, T, N, FGPow) X(P, T, N, FRProd)     \
     X(P, T, N, FRProdE) X(P, T, N, FRE) X(P, T, N, FUGradU) X(P, T, N, FDot3) X(P, T, N, FEDot)                   \
-    X(P, T, N, FRProd2) X(P, T, N, FRProd2E) X(P, T, N, FG1) X(P, T, N, FG2) X(P, T, N, FG2E) X(P, T, N, FG2T)    \
+    X(P, T, N, FRTrial<false>) X(P, T, N, FRTrial<true>) X(P, T, N, FRTrialE) X(P, T, N, FG1) X(P, T, N, FG2) X(P, T, N, FG2E) X(P, T, N, FG2T)    \
     X(P, T, N, FG3<false>) X(P, T, N, FG3<true>) X(P, T, N, FC3) X(P, T, N, FLSS) X(P, T, N, FLSS12)              \
     X(P, T, N, FLSW<0>) X(P, T, N, FLSW<1>) X(P, T, N, FLSQG) X(P, T, N, FLSA) X(P, T, N, FAPow)           \
     X(P, T, N, FLSE) X(P, T, N, FLSTrial<false>) X(P, T, N, FLSTrial<true>)                               \

@@ -207,27 +207,43 @@ struct FRRed1 {
     }
 };
 
-// general q >= 4: forward outputs sum V^2, p*a4, u.V.  inputs V(3), p, u(3), a4
-struct FRProd2 {
-    static constexpr int NIN = 8, NOUT = 3, NRED = 0;
+// q branch of R: out p a4 and u . V, and the R1 and R2 integrands A a4 G and
+// a4 sum V^2; with RAW also sum V^2 and a4 (FLSTrial, which is this along a
+// line, says which products need no transform).  inputs V(3), p, u(3), a4, A, G
+template <bool RAW>
+struct FRTrial {
+    static constexpr int NIN = 10, NOUT = RAW ? 4 : 2, NRED = RAW ? 1 : 2;
+    int direct;
     template <typename T>
-    __device__ void operator()(const T* in, T* out, double*) const {
-        out[0] = in[0] * in[0] + in[1] * in[1] + in[2] * in[2];
-        out[1] = in[3] * in[7];
-        out[2] = in[4] * in[0] + in[5] * in[1] + in[6] * in[2];
+    __device__ void operator()(const T* in, T* out, double* acc) const {
+        const T v2 = in[0] * in[0] + in[1] * in[1] + in[2] * in[2];
+        const T a4 = in[7], a = in[8];
+        out[0] = in[3] * a4;
+        out[1] = in[4] * in[0] + in[5] * in[1] + in[6] * in[2];
+        acc[0] += (double)(direct ? a : a * a4) * (double)in[9];
+        if constexpr (RAW) {
+            out[2] = v2;
+            out[3] = a4;
+        } else {
+            acc[1] += (double)a4 * (double)v2;
+        }
     }
 };
 
-// e_u branch: sum E^2, p*a2, e.E.  inputs E(3), p, u(3), S, a2
-struct FRProd2E {
-    static constexpr int NIN = 9, NOUT = 3, NRED = 0;
+// e_u branch of R: out sum E^2, p a2, e . E and a2, and the R1 integrand a2 G.
+// inputs E(3), p, u(3), S, a2, G
+struct FRTrialE {
+    static constexpr int NIN = 10, NOUT = 4, NRED = 1;
     template <typename T>
-    __device__ void operator()(const T* in, T* out, double*) const {
+    __device__ void operator()(const T* in, T* out, double* acc) const {
         T e[3];
         unit_vec(in + 4, in[7], e);
+        const T a2 = in[8];
         out[0] = in[0] * in[0] + in[1] * in[1] + in[2] * in[2];
-        out[1] = in[3] * in[8];
+        out[1] = in[3] * a2;
         out[2] = e[0] * in[0] + e[1] * in[1] + e[2] * in[2];
+        out[3] = a2;
+        acc[0] += (double)a2 * (double)in[9];
     }
 };
 
