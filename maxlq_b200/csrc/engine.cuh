@@ -25,11 +25,8 @@ namespace mlq {
 // launchers of the device line search's kernels (lsdev.cu)
 void ls_launch_coef(LsDevState* s, const double* results, const double* partials, int nblocks, const LsAnchorSet& an,
                     cudaStream_t st);
-void ls_launch_ctrl(LsDevState* s, cudaGraphConditionalHandle h_loop, cudaGraphConditionalHandle h_chk,
-                    cudaStream_t st);
-void ls_launch_check(LsDevState* s, const double* partials, int nblocks, cudaGraphConditionalHandle h_fft,
-                     cudaStream_t st);
-void ls_launch_fft(LsDevState* s, const double* r, cudaStream_t st);
+void ls_launch_ctrl(LsDevState* s, const double* r, int direct, cudaGraphConditionalHandle h_loop,
+                    cudaGraphConditionalHandle h_next, cudaStream_t st);
 
 // A state vector: three components of nb*nb*nx Fourier coefficients of band
 // b2, stored as double2 (FP64 path) or float2 (the mixed path's FP32 state);
@@ -518,6 +515,13 @@ class Engine : public EngineBase {
     // 0: the search ran (out filled); 1: not available, search on the host
     int ls_device_search(double B, double tA0, double tB0, LsOut* out);
     bool ls_graph_build(LsGraph& g, int key);
+    // A tau outside the clamp-free intervals takes the transform without the
+    // check of S(tau) >= 0 before it: at n <= 64 the check costs as much as
+    // the transform (two kernels and a conditional node against three), and on
+    // such grids it mostly fails.  FP64 only: in FP32 the value of a transform
+    // carries noise that the polynomial of a passed check does not.
+    // A 32^3 q = 4 iteration, with some ten such trials: 0.66 -> 0.62 ms.
+    bool ls_direct() const { return sizeof(T) == 8 && n <= 64; }
 
     // ---- state <-> host ----
     // Forward transform of a host FP64 vector field into state spectra.

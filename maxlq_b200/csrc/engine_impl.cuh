@@ -2659,6 +2659,48 @@ void Engine<T>::ls_setup(const SVec* u, const SVec* d, double tau0) {
     ls_host_poly_ = true;
 }
 
+// ls_min_kernel at the search's ptau, whose last block to finish decides: the
+// transform branch opens unless S(ptau) >= 0 at every point.
+template <typename T>
+__global__ void __launch_bounds__(RED_THREADS)
+    ls_min_check_kernel(const T* __restrict__ s0, const T* __restrict__ s1, const T* __restrict__ s2, long npts,
+                        LsDevState* st, double* out, cudaGraphConditionalHandle h_fft) {
+    const T t = (T)st->ptau;
+    T m = T(1e30);
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < npts; i += (long)gridDim.x * blockDim.x)
+        m = fmin(m, s0[i] + t * (s1[i] + t * s2[i]));
+    __shared__ T sm[RED_THREADS / 32];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto block_min = [&](T v) {  // in thread 0
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_down_sync(0xffffffffu, v, o));
+        if (lane == 0) sm[warp] = v;
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = fmin(v, sm[w]);
+        return v;
+    };
+    m = block_min(m);
+    if (threadIdx.x == 0) {
+        __stcg(out + blockIdx.x, (double)m);
+        __threadfence();
+        last = atomicAdd(&st->checked, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    T v = T(1e30);
+    for (int g = threadIdx.x; g < (int)gridDim.x; g += blockDim.x) v = fmin(v, (T)__ldcg(out + g));
+    v = block_min(v);
+    if (threadIdx.x == 0) {
+        const bool free_tau = v >= T(0) && !st->par.transform_trials;
+        st->checked = 0;
+        st->need = free_tau ? 3 : 2;
+        cudaGraphSetConditional(h_fft, free_tau ? 0 : 1);
+    }
+}
+
 template <typename T>
 void Engine<T>::ls_poly_to_host() {
     if (ls_host_poly_) return;
@@ -2703,7 +2745,9 @@ static cudaGraph_t add_conditional(cudaGraph_t g, cudaGraphNode_t dep, cudaGraph
 }
 
 // The device search as one graph:
-//   while (h_loop) { ctrl; if (h_chk) { ls_min; check; if (h_fft) { transform trial; fft } } }
+//   while (h_loop) { ctrl; if (h_chk) { check; if (h_fft) { transform trial } } }
+// or, where no check comes before the transform (ls_direct),
+//   while (h_loop) { ctrl; if (h_chk) { transform trial } }
 // Each conditional handle is set by a kernel of the graph that holds its node
 // (the loop's by the controller in its body).  The controller ends the loop
 // after LS_MAX_LOOPS passes, so the loop is bounded whatever the kernels see.
@@ -2757,22 +2801,27 @@ bool Engine<T>::ls_graph_build(LsGraph& g, int key) {
             MLQ_CUDA(cudaGraphConditionalHandleCreate(&h_loop, G, 1, cudaGraphCondAssignDefault));
             cudaGraph_t body_loop = add_conditional(G, nullptr, h_loop, cudaGraphCondTypeWhile);
             MLQ_CUDA(cudaGraphConditionalHandleCreate(&h_chk, body_loop, 0, cudaGraphCondAssignDefault));
-            capture_into(body_loop, [&] { ls_launch_ctrl(d_ls_, h_loop, h_chk, stream); });
-            cudaGraph_t body_chk = add_conditional(body_loop, graph_leaf(body_loop), h_chk, cudaGraphCondTypeIf);
-            MLQ_CUDA(cudaGraphConditionalHandleCreate(&h_fft, body_chk, 0, cudaGraphCondAssignDefault));
-            capture_into(body_chk, [&] {
-                launch_k(ls_min_kernel<T>, grid, RED_THREADS, 0, phys(in[0]), phys(in[1]), phys(in[2]), n3, 0.0,
-                                                                   &d_ls_->ptau, d_partials);
-                ls_launch_check(d_ls_, d_partials, grid, h_fft, stream);
+            capture_into(body_loop, [&] {
+                ls_launch_ctrl(d_ls_, d_results + 130, ls_direct() ? 1 : 0, h_loop, h_chk, stream);
             });
-            cudaGraph_t body_fft = add_conditional(body_chk, graph_leaf(body_chk), h_fft, cudaGraphCondTypeIf);
-            capture_into(body_fft, [&] {
+            cudaGraph_t body_chk = add_conditional(body_loop, graph_leaf(body_loop), h_chk, cudaGraphCondTypeIf);
+            auto transform = [&] {
                 FLSA f;
                 f.tau = 0.0;
                 f.taup = &d_ls_->ptau;
                 fwd(b2, f, in, {o}, 130);
-                ls_launch_fft(d_ls_, d_results + 130, stream);
-            });
+            };
+            if (ls_direct()) {
+                capture_into(body_chk, transform);
+            } else {
+                MLQ_CUDA(cudaGraphConditionalHandleCreate(&h_fft, body_chk, 0, cudaGraphCondAssignDefault));
+                capture_into(body_chk, [&] {
+                    ls_min_check_kernel<T><<<grid, RED_THREADS, 0, stream>>>(phys(in[0]), phys(in[1]), phys(in[2]), n3,
+                                                                             d_ls_, d_partials, h_fft);
+                });
+                cudaGraph_t body_fft = add_conditional(body_chk, graph_leaf(body_chk), h_fft, cudaGraphCondTypeIf);
+                capture_into(body_fft, transform);
+            }
             MLQ_CUDA(cudaGraphInstantiate(&exec, G, 0));
         } catch (...) {
             ok = false;
@@ -2828,7 +2877,7 @@ int Engine<T>::ls_device_search(double B, double tA0, double tB0, LsOut* out) {
     ls_host_poly_ = true;
     *out = *ho;
     // the graph's kernels (one launch counted above)
-    launches += out->loops + 2LL * out->checks + out->nfft * (g->nfwd + 1) - 1;
+    launches += out->loops + (long long)out->checks + out->nfft * g->nfwd - 1;
     ++ls_dev_searches_;
     ls_dev_loops_ += out->loops;
     ls_poly_trials_ += out->npoly;
@@ -2846,7 +2895,7 @@ bool Engine<T>::ls_clamp_free(double tau) {
     if (ls_transform_trials_) return false;
     ls_poly_to_host();
     bool clamp_off = ls_free(ls_c_, tau);
-    if (!clamp_off) {
+    if (!clamp_off && !(ls_ok() && ls_direct())) {
         // outside the interval: one read of S_0..2 decides for this tau
         const long npts = slab_ ? (long)zs_ * n * n : n3;
         const int grid = grid_for(npts, RED_THREADS, 148 * 4);

@@ -386,7 +386,8 @@ struct LsDevState {
     LsParams par;
     LsOut out;
     int ntr;
-    int need;  // 0 none, 1 check of ptau pending, 2 transform of ptau pending
+    int need;  // 0 none, 1 check of ptau pending, 2 transform of ptau ran, 3 ptau is clamp-free
+    unsigned checked;  // blocks of the check that are done
     double ptau;
     double mtau[LS_MEMO], mR[LS_MEMO][3], mlqq[LS_MEMO], mJ[LS_MEMO];
     int mfft[LS_MEMO];

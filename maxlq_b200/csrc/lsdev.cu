@@ -129,20 +129,37 @@ __global__ void __launch_bounds__(LS_COEF_THREADS)
     ls_assemble(results + 100, results + 140, results + 149, lo[0], hi[0], lo + 1, hi + 1, an.a, s->poly);
     s->ntr = 0;
     s->need = 0;
+    s->checked = 0;
     s->ptau = 0.0;
     s->out = LsOut{};
     s->out.status = LS_RUNNING;
 }
 
-// One pass of the controller: mnbrak then Brent from the start over the
-// table; ends the loop when the search completes (or fails), else leaves
-// the first tau without a value in ptau and opens the check branch.
-__global__ void ls_ctrl_kernel(LsDevState* s, cudaGraphConditionalHandle h_loop, cudaGraphConditionalHandle h_chk) {
+// One pass of the controller: the value of the last tau, then mnbrak and Brent
+// from the start over the table; ends the loop when the search completes (or
+// fails), else leaves the first tau without a value in ptau and opens the
+// branch h_next (the check, or with `direct` the transform).  sums: those of a
+// transform trial.
+__global__ void ls_ctrl_kernel(LsDevState* s, const double* __restrict__ sums, int direct,
+                               cudaGraphConditionalHandle h_loop, cudaGraphConditionalHandle h_next) {
     __shared__ LsShared sh;
-    const int n = s->ntr;
     for (int i = threadIdx.x; i < (int)(sizeof(LsPoly) / sizeof(double)); i += blockDim.x)
         reinterpret_cast<double*>(&sh.poly)[i] = reinterpret_cast<const double*>(&s->poly)[i];
-    if (threadIdx.x == 0) sh.par = s->par;
+    if (threadIdx.x == 0) {
+        sh.par = s->par;
+        if (s->need >= 2) {
+            const LsParams& p = s->par;
+            double R[3], lqq;
+            if (s->need == 2)
+                ls_fft_R(s->poly, p.q, p.cv, p.cp, sums, s->ptau, R, &lqq);
+            else
+                ls_poly_R(s->poly, p.q, p.cv, p.cp, s->ptau, R, &lqq);
+            if (!ls_memo_add(s, s->ptau, R, lqq, s->need == 2)) s->out.status = LS_ERR_CAP;
+            s->need = 0;
+        }
+    }
+    __syncwarp();
+    const int n = s->ntr;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         sh.tau[i] = s->mtau[i];
         sh.J[i] = s->mJ[i];
@@ -151,11 +168,11 @@ __global__ void ls_ctrl_kernel(LsDevState* s, cudaGraphConditionalHandle h_loop,
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     LsOut& o = s->out;
     if (o.status != LS_RUNNING) {
-        ls_stop(s, o.status, h_loop, h_chk);
+        ls_stop(s, o.status, h_loop, h_next);
         return;
     }
     if (o.loops >= LS_MAX_LOOPS) {
-        ls_stop(s, LS_ERR_CAP, h_loop, h_chk);
+        ls_stop(s, LS_ERR_CAP, h_loop, h_next);
         return;
     }
     ++o.loops;
@@ -165,15 +182,15 @@ __global__ void ls_ctrl_kernel(LsDevState* s, cudaGraphConditionalHandle h_loop,
     int r = ls_mnbrak(ev, s->par.tA0, s->par.tB0, tb, &mflag);
     if (r == 0) r = ls_brent(ev, tb, &x, &fx);
     if (ev.err) {
-        ls_stop(s, ev.err, h_loop, h_chk);
+        ls_stop(s, ev.err, h_loop, h_next);
         return;
     }
     if (r == LS_SUSPEND) {
-        s->need = 1;
+        s->need = direct ? 2 : 1;
         s->ptau = ev.ptau;
-        ++o.checks;
+        if (!direct) ++o.checks;
         cudaGraphSetConditional(h_loop, 1);
-        cudaGraphSetConditional(h_chk, 1);
+        cudaGraphSetConditional(h_next, 1);
         return;
     }
     o.mflag = mflag;
@@ -197,51 +214,16 @@ __global__ void ls_ctrl_kernel(LsDevState* s, cudaGraphConditionalHandle h_loop,
                 break;
             }
     }
-    ls_stop(s, 0, h_loop, h_chk);
-}
-
-// After the minimum of S(ptau) over the points (per-block minima in
-// partials): the polynomial value where S >= 0 everywhere, else open the
-// transform branch.
-__global__ void ls_check_kernel(LsDevState* s, const double* __restrict__ partials, int nblocks,
-                                cudaGraphConditionalHandle h_fft) {
-    double mn = 1e300;
-    for (int g = threadIdx.x; g < nblocks; g += 32) mn = fmin(mn, partials[g]);
-    for (int o = 16; o > 0; o >>= 1) mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (mn >= 0.0 && !s->par.transform_trials) {
-        double R[3], lqq;
-        ls_poly_R(s->poly, s->par.q, s->par.cv, s->par.cp, s->ptau, R, &lqq);
-        if (!ls_memo_add(s, s->ptau, R, lqq, 0)) s->out.status = LS_ERR_CAP;
-        s->need = 0;
-        cudaGraphSetConditional(h_fft, 0);
-    } else {
-        s->need = 2;
-        cudaGraphSetConditional(h_fft, 1);
-    }
-}
-
-// After the transform trial at ptau: its sums r[0..3] give the value.
-__global__ void ls_fft_kernel(LsDevState* s, const double* __restrict__ r) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double R[3], lqq;
-    ls_fft_R(s->poly, s->par.q, s->par.cv, s->par.cp, r, s->ptau, R, &lqq);
-    if (!ls_memo_add(s, s->ptau, R, lqq, 1)) s->out.status = LS_ERR_CAP;
-    s->need = 0;
+    ls_stop(s, 0, h_loop, h_next);
 }
 
 void ls_launch_coef(LsDevState* s, const double* results, const double* partials, int nblocks, const LsAnchorSet& an,
                     cudaStream_t st) {
     MLQ_CUDA(launch_pdl(true, ls_coef_kernel, 1, LS_COEF_THREADS, 0, st, s, results, partials, nblocks, an));
 }
-void ls_launch_ctrl(LsDevState* s, cudaGraphConditionalHandle h_loop, cudaGraphConditionalHandle h_chk,
-                    cudaStream_t st) {
-    ls_ctrl_kernel<<<1, 32, 0, st>>>(s, h_loop, h_chk);
+void ls_launch_ctrl(LsDevState* s, const double* r, int direct, cudaGraphConditionalHandle h_loop,
+                    cudaGraphConditionalHandle h_next, cudaStream_t st) {
+    ls_ctrl_kernel<<<1, 32, 0, st>>>(s, r, direct, h_loop, h_next);
 }
-void ls_launch_check(LsDevState* s, const double* partials, int nblocks, cudaGraphConditionalHandle h_fft,
-                     cudaStream_t st) {
-    ls_check_kernel<<<1, 32, 0, st>>>(s, partials, nblocks, h_fft);
-}
-void ls_launch_fft(LsDevState* s, const double* r, cudaStream_t st) { ls_fft_kernel<<<1, 32, 0, st>>>(s, r); }
 
 }  // namespace mlq
