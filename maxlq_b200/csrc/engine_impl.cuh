@@ -199,14 +199,31 @@ void Engine<T>::zfwd_cv(ZFwdArgs<T>& za, int narr) {
             using PS = PairShape<NN>;
             const size_t smem = PS::SMEM + 2 * NN * sizeof(float);  // + the K table
             const long items = (long)za.band.nb * (((za.nx + 1) / 2 + PS::NP - 1) / PS::NP);
-            auto kern = zfwd_pair_kernel<NN, YShape<NN, T, V>::PAIR_MINB>;
-            allow_smem(kern);
-            const int G = persistent_blocks((const void*)kern, PS::THREADS, smem);
-            dim3 grid((unsigned)std::min<long>(items, std::max(1, G / narr)), narr);
-            last_zblocks_ = (long)grid.x * narr;
-            ensure_partials(last_zblocks_ * MAX_RED);
-            za.partials = d_partials;
-            this->launch_k(kern, grid, PS::THREADS, smem, za, d_twT_ + tw_off.at(NN));
+            bool add = false, red = false, rt = false;
+            for (int i = 0; i < narr; ++i) {
+                const ZFwdOp& op = za.op[i];
+                add = add || op.add;
+                red = red || op.red_self >= 0 || op.red_with[0] || op.red_with[1] || op.red_with[2];
+                rt = rt || op.ys_out;
+            }
+            auto run = [&](auto kern) {
+                allow_smem(kern);
+                const int G = persistent_blocks((const void*)kern, PS::THREADS, smem);
+                dim3 grid((unsigned)std::min<long>(items, std::max(1, G / narr)), narr);
+                last_zblocks_ = (long)grid.x * narr;
+                ensure_partials(last_zblocks_ * MAX_RED);
+                za.partials = d_partials;
+                this->launch_k(kern, grid, PS::THREADS, smem, za, d_twT_ + tw_off.at(NN));
+            };
+            constexpr int MINB = YShape<NN, T, V>::PAIR_MINB;
+            if (!add && !red)
+                run(zfwd_pair_kernel<NN, MINB, ZK_PLAIN>);
+            else if (!red && !rt)
+                run(zfwd_pair_kernel<NN, MINB, ZK_ADD>);
+            else if (!add && !rt)
+                run(zfwd_pair_kernel<NN, MINB, ZK_RED>);
+            else
+                run(zfwd_pair_kernel<NN, MINB, ZK_ALL>);
         }
         return;
     }
