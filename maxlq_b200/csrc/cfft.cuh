@@ -455,6 +455,13 @@ __device__ __forceinline__ void block_reduce_to(const double* acc, double* out) 
 // ----------------------------------------------------------------------------
 // x stage, inverse (c2r).  grid = (G, narr), block = XTHREADS.  Each block
 // walks groups of XTHREADS/TPL lines of array blockIdx.y.
+//
+// A field and its x derivative differ by the factor i kx of the last stage
+// alone, so both come from one x-stage array: the line is read again (from
+// L1), multiplied and transformed for the second output.  That takes the z
+// and y passes and the arrays of d_x off every (field, gradient) family and off
+// the d_x S of a round trip: of an iteration's 36 inverse transforms 5
+// through the x stage alone.  DXFIG
 // ----------------------------------------------------------------------------
 template <int N, typename T>
 __global__ void __launch_bounds__(CShape<N, T>::XTHREADS, 512 / CShape<N, T>::XTHREADS)
@@ -476,6 +483,13 @@ __global__ void __launch_bounds__(CShape<N, T>::XTHREADS, 512 / CShape<N, T>::XT
         tw.tab = stw;
     }
     const cpx<T> wt = twN[t];  // W_N^t
+    __shared__ T kx[L];  // 2 pi k, rounded once as in the z stage
+    const int nrep = a.dx[blockIdx.y] ? 2 : 1;
+    if (nrep == 2) {
+        for (int i = threadIdx.x; i < L; i += blockDim.x)
+            kx[i] = (T)(2.0 * 3.14159265358979311600 * (double)i);
+        __syncthreads();
+    }
     pdl_begin<(N <= 64)>();
     const int nx_in = a.nx_in;
     const int px = a.px ? a.px : nx_in;  // row pitch of xs
@@ -485,37 +499,44 @@ __global__ void __launch_bounds__(CShape<N, T>::XTHREADS, 512 / CShape<N, T>::XT
     for (long g = blockIdx.x; g < NG; g += gridDim.x) {
         const long line = g * LPB + ls;
         const cpx<T>* __restrict__ src = src0 + line * px;
-        cpx<T> v[E];
+#pragma unroll 1
+        for (int rep = 0; rep < nrep; ++rep) {
+            cpx<T> v[E];
 #pragma unroll
-        for (int m = 0; m < E; ++m) {
-            const int k = t + TPL * m;
-            v[m] = k < nx_in ? src[k] : czero<T>();
-        }
-        // c2c + REAL() keeps the Hermitian part: real part only on kx = 0, N/2
-        cpx<T> xh = czero<T>();
-        if (t == 0) {
-            v[0].y = T(0);
-            if (L < nx_in) xh = mk(src[L].x, T(0));
-        }
-        cpx<T> o[E];
-        SFor<0, E>::run([&](auto mc) {
-            constexpr int m = decltype(mc)::value;
-            cpx<T> xp;  // X[L - k], k = t + TPL m
-            xp.x = __shfl_sync(0xffffffffu, v[E - 1 - m].x, src_lane, TPL);
-            xp.y = __shfl_sync(0xffffffffu, v[E - 1 - m].y, src_lane, TPL);
-            if (t == 0) xp = (m == 0) ? xh : v[(E - m) % E];
-            const cpx<T> xk = v[m];
-            const cpx<T> xc = conj(xp);
-            const cpx<T> Fk = xk + xc;
-            // G = (xk - xc) * conj(W_N^k),  W_N^k = W_N^t * W_N^(TPL m)
-            const cpx<T> w = wt * cw<T, N, (long)TPL * m>();
-            const cpx<T> G = cmul_s<+1>(xk - xc, w);
-            o[m] = mk(Fk.x - G.y, Fk.y + G.x);  // F + i G
-        });
-        cfft<L, E, +1, SyncWarp>(o, t, sm, map, tw);
-        cpx<T>* __restrict__ dst = reinterpret_cast<cpx<T>*>(dst0 + line * N);
+            for (int m = 0; m < E; ++m) {
+                const int k = t + TPL * m;
+                v[m] = k < nx_in ? src[k] : czero<T>();
+                if (rep) {
+                    const T f = (T)a.dx_coef[blockIdx.y] * kx[k];
+                    v[m] = mk(-f * v[m].y, f * v[m].x);
+                }
+            }
+            // c2c + REAL() keeps the Hermitian part: real part only on kx = 0, N/2
+            cpx<T> xh = czero<T>();
+            if (t == 0) {
+                v[0].y = T(0);
+                if (L < nx_in && !rep) xh = mk(src[L].x, T(0));  // an odd factor vanishes at N/2
+            }
+            cpx<T> o[E];
+            SFor<0, E>::run([&](auto mc) {
+                constexpr int m = decltype(mc)::value;
+                cpx<T> xp;  // X[L - k], k = t + TPL m
+                xp.x = __shfl_sync(0xffffffffu, v[E - 1 - m].x, src_lane, TPL);
+                xp.y = __shfl_sync(0xffffffffu, v[E - 1 - m].y, src_lane, TPL);
+                if (t == 0) xp = (m == 0) ? xh : v[(E - m) % E];
+                const cpx<T> xk = v[m];
+                const cpx<T> xc = conj(xp);
+                const cpx<T> Fk = xk + xc;
+                // G = (xk - xc) * conj(W_N^k),  W_N^k = W_N^t * W_N^(TPL m)
+                const cpx<T> w = wt * cw<T, N, (long)TPL * m>();
+                const cpx<T> G = cmul_s<+1>(xk - xc, w);
+                o[m] = mk(Fk.x - G.y, Fk.y + G.x);  // F + i G
+            });
+            cfft<L, E, +1, SyncWarp>(o, t, sm, map, tw);
+            cpx<T>* __restrict__ dst = reinterpret_cast<cpx<T>*>((rep ? a.dx[blockIdx.y] : dst0) + line * N);
 #pragma unroll
-        for (int m = 0; m < E; ++m) dst[t + TPL * m] = o[m];
+            for (int m = 0; m < E; ++m) dst[t + TPL * m] = o[m];
+        }
     }
 }
 

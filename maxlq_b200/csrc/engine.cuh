@@ -384,6 +384,8 @@ class Engine : public EngineBase {
         void* spec = nullptr;
         int spec_f64 = 0;
         int phys_out = -1;   // round trip destination (phys index), -1 none
+        int dx_out = -1;     // and dx_coef d_x of it (share_dx only)
+        double dx_coef = 0.0;
         int sym = SYM_ONE, ab = 0;
         const void* add = nullptr;
         int add_f64 = 0, add_sym = SYM_ONE, add_ab = 0;
@@ -402,7 +404,11 @@ class Engine : public EngineBase {
         ZSrc src[3];
         int nsrc = 0;
         int phys_out = -1;
+        int dx_out = -1;  // dx_coef d_x of the output, from the same x-stage array
+        double dx_coef = 0.0;
     };
+    // x derivatives from the x stage of their field (xinv_c_kernel)
+    bool share_dx() const { return cfft_ok_ && reuse_on_ && !slab_; }
     void inv(const Band& b, const std::vector<InvOut>& outs);
     template <int NOUT>
     void fwd_z(const Band& b, const std::vector<FwdOut>& outs, int red_dst, double norm);
@@ -411,7 +417,11 @@ class Engine : public EngineBase {
                   int fred_dst, double norm);
     template <class F>
     void pointwise(const F& f, const std::vector<int>& in, const std::vector<int>& out, int fred_dst = -1);
-    void yx_inverse(const Band& b, const std::vector<cpx<T>*>& ys, const std::vector<int>& phys_out);
+    struct PhysOut {
+        int phys, dx;
+        double dx_coef;
+    };
+    void yx_inverse(const Band& b, const std::vector<cpx<T>*>& ys, const std::vector<PhysOut>& out);
 
     // ---- programs ----
     // R parts at phi = u + tau*d (d may be null) -> results; also ||phi||_q^q.
@@ -469,6 +479,7 @@ class Engine : public EngineBase {
     // parts of the setups
     struct LsFields {
         std::vector<int> ud, all, grads;  // u, d; u, Du, d, Dd; Du, Dd
+        bool vx[3] = {false, false, false};  // V_a0 formed with S_a
     };
     LsFields ls_fields(const SVec* u, const SVec* d);
     void ls_w_fields(const LsFields& lf);

@@ -796,7 +796,9 @@ void Engine<T>::launch_xinv(XInvArgs<T>& xa, int narr, const Band& b) {
     xa.px = px_of(b);
     const int h = n / 2;
     if (xa.nlines <= 0) xa.nlines = (long)n * n;
-    const double bytes = (double)narr * xa.nlines * ((double)b.nx * sizeof(cpx<T>) + (double)n * sizeof(T));
+    double bytes = (double)narr * xa.nlines * ((double)b.nx * sizeof(cpx<T>) + (double)n * sizeof(T));
+    for (int i = 0; i < narr; ++i)
+        if (xa.dx[i]) bytes += (double)xa.nlines * n * sizeof(T);
     xa.tw_n_off = tw_off.at(n);
     if (cfft_ok_) {
         cudaEvent_t ev = prof_mark();
@@ -1001,18 +1003,18 @@ void Engine<T>::fwd_z(const Band& b, const std::vector<FwdOut>& outs, int red_ds
     }
     if (any_rt) {
         std::vector<cpx<T>*> ys;
-        std::vector<int> po;
+        std::vector<PhysOut> po;
         for (int o = 0; o < NOUT; ++o)
             if (outs[o].phys_out >= 0) {
                 ys.push_back(ysbuf(o));
-                po.push_back(outs[o].phys_out);
+                po.push_back({outs[o].phys_out, outs[o].dx_out, outs[o].dx_coef});
             }
         yx_inverse(b, ys, po);
     }
 }
 
 template <typename T>
-void Engine<T>::yx_inverse(const Band& b, const std::vector<cpx<T>*>& ys, const std::vector<int>& phys_out) {
+void Engine<T>::yx_inverse(const Band& b, const std::vector<cpx<T>*>& ys, const std::vector<PhysOut>& out) {
     const int k = (int)ys.size();
     if (k == 0) return;
     // y inverse: ys[i] -> xs (xs buffers are free once the forward's y pass ran)
@@ -1033,8 +1035,13 @@ void Engine<T>::yx_inverse(const Band& b, const std::vector<cpx<T>*>& ys, const 
     xa.nx_in = b.nx;
     for (int i = 0; i < k; ++i) {
         xa.in[i] = xs[i];
-        xa.out[i] = phys(phys_out[i]);
-        phys_written(phys_out[i]);
+        xa.out[i] = phys(out[i].phys);
+        phys_written(out[i].phys);
+        if (out[i].dx >= 0) {
+            xa.dx[i] = phys(out[i].dx);
+            xa.dx_coef[i] = out[i].dx_coef;
+            phys_written(out[i].dx);
+        }
     }
     xa.plan_half = plan(n / 2);
     xa.tw = d_tw;
@@ -1042,14 +1049,36 @@ void Engine<T>::yx_inverse(const Band& b, const std::vector<cpx<T>*>& ys, const 
 }
 
 template <typename T>
-void Engine<T>::inv(const Band& b, const std::vector<InvOut>& outs) {
+void Engine<T>::inv(const Band& b, const std::vector<InvOut>& all) {
     if (b.nx > nxcap || b.nb > nbcap) throw CudaError("inv: band exceeds buffers", MLQ_ERR_BADARG);
     const int G = 6;
     bool multi = cfft_ok_ && multi_zinv_;
-    for (const InvOut& io : outs) multi = multi && io.nsrc == 1;
+    for (const InvOut& io : all) multi = multi && io.nsrc == 1;
+    auto same_source = [](const InvOut& x, const InvOut& y) {
+        return x.nsrc == 1 && y.nsrc == 1 && x.src[0].spec == y.src[0].spec && x.src[0].f64 == y.src[0].f64;
+    };
+    // the x derivative that follows its field comes from the field's x stage
+    std::vector<InvOut> outs;
+    for (const InvOut& io : all) {
+        if (share_dx() && !outs.empty() && same_source(outs.back(), io) && outs.back().dx_out < 0 &&
+            outs.back().src[0].sym == SYM_ONE && io.src[0].sym == SYM_IKX) {
+            outs.back().dx_out = io.phys_out;
+            outs.back().dx_coef = io.src[0].coef / outs.back().src[0].coef;
+        } else {
+            outs.push_back(io);
+        }
+    }
     const size_t GM = multi ? MAX_ARR : G;
-    for (size_t g0 = 0; g0 < outs.size(); g0 += GM) {
-        const int k = (int)std::min<size_t>(GM, outs.size() - g0);
+    size_t step = 0;
+    for (size_t g0 = 0; g0 < outs.size(); g0 += step) {
+        // whole families of one source per launch, where they fit
+        step = std::min<size_t>(GM, outs.size() - g0);
+        if (g0 + step < outs.size()) {
+            size_t e = step;
+            while (e > 1 && same_source(outs[g0 + e], outs[g0 + e - 1])) --e;
+            if (e > 1 || !same_source(outs[g0 + 1], outs[g0])) step = e;
+        }
+        const int k = (int)step;
         if (multi) {
             // consecutive outputs of one source spectrum share a load
             ZInvMultiArgs<T> zm;
@@ -1057,7 +1086,7 @@ void Engine<T>::inv(const Band& b, const std::vector<InvOut>& outs) {
             zm.nx = b.nx;
             zm.band = b;
             std::vector<cpx<T>*> ys(k);
-            std::vector<int> po(k);
+            std::vector<PhysOut> po(k);
             int nops = 0;
             double zb = 0;
             for (int i = 0; i < k; ++i) {
@@ -1076,13 +1105,13 @@ void Engine<T>::inv(const Band& b, const std::vector<InvOut>& outs) {
                 op->coef[o] = io.src[0].coef;
                 ys[i] = slab_ ? slot_ys(io.phys_out) : ysbuf(i);
                 op->ys_out[o] = ys[i];
-                po[i] = io.phys_out;
+                po[i] = {io.phys_out, io.dx_out, io.dx_coef};
                 zb += (double)n * b.nb * b.nx * sizeof(cpx<T>);
             }
             launch_zinv_multi(zm, nops, b, zb);
             if (slab_) {
                 for (int i = 0; i < k; ++i) {
-                    PSlot& sl = slot(po[i]);
+                    PSlot& sl = slot(po[i].phys);
                     sl.kind = PSlot::YS;
                     sl.band = b;
                 }
@@ -1096,7 +1125,7 @@ void Engine<T>::inv(const Band& b, const std::vector<InvOut>& outs) {
         za.nx = b.nx;
         za.band = b;
         std::vector<cpx<T>*> ys(k);
-        std::vector<int> po(k);
+        std::vector<PhysOut> po(k);
         for (int i = 0; i < k; ++i) {
             const InvOut& io = outs[g0 + i];
             ZInvOp& op = za.op[i];
@@ -1104,7 +1133,7 @@ void Engine<T>::inv(const Band& b, const std::vector<InvOut>& outs) {
             op.nsrc = io.nsrc;
             ys[i] = slab_ ? slot_ys(io.phys_out) : ysbuf(i);
             op.ys_out = ys[i];
-            po[i] = io.phys_out;
+            po[i] = {io.phys_out, io.dx_out, io.dx_coef};
         }
         double zb = 0;
         for (int i = 0; i < k; ++i) {
@@ -1115,7 +1144,7 @@ void Engine<T>::inv(const Band& b, const std::vector<InvOut>& outs) {
         launch_zinv(za, k, b, zb);
         if (slab_) {
             for (int i = 0; i < k; ++i) {
-                PSlot& sl = slot(po[i]);
+                PSlot& sl = slot(po[i].phys);
                 sl.kind = PSlot::YS;
                 sl.band = b;
             }
@@ -1740,9 +1769,13 @@ void Engine<T>::R_eval(const SVec* u, const SVec* d, double tau, double out[3], 
         // one spectrum instead of three round trips
         oS.spec = wspec(WRS);
         oS.spec_f64 = wf64<T>();
+        if (share_dx()) {
+            oS.dx_out = PV;
+            oS.dx_coef = 0.5;
+        }
         fwd(b, FRProdE{}, uin, {oS, oQ, oG2});
         std::vector<InvOut> g;
-        for (int j = 0; j < 3; ++j) {
+        for (int j = share_dx() ? 1 : 0; j < 3; ++j) {
             InvOut o;
             o.nsrc = 1;
             o.src[0] = ZSrc{wspec(WRS), wf64<T>(), SYM_IKX + j, 0, 0.5};
@@ -2473,6 +2506,11 @@ typename Engine<T>::LsFields Engine<T>::ls_fields(const SVec* u, const SVec* d) 
         o[a].phys_out = LS + a;
         o[a].spec = wspec(WLS + a);
         o[a].spec_f64 = wf64<T>();
+        if (share_dx() && !use_e_u && 3 * b2.cut < n && (a > 0 || !s0)) {
+            o[a].dx_out = LV + 3 * a;  // V_a0 = (1/2) d_x S_a (ls_w_fields)
+            o[a].dx_coef = 0.5;
+            lf.vx[a] = true;
+        }
     }
     if (s0)
         fwd(b2, FLSS12{}, lf.ud, {o[1], o[2]});
@@ -2493,7 +2531,7 @@ void Engine<T>::ls_w_fields(const LsFields& lf) {
     if (reuse_on_ && 3 * b2.cut < n) {
         std::vector<InvOut> g;
         for (int a = 0; a < 3; ++a)
-            for (int j = 0; j < 3; ++j) {
+            for (int j = lf.vx[a] ? 1 : 0; j < 3; ++j) {
                 InvOut o;
                 o.nsrc = 1;
                 o.src[0] = ZSrc{wspec(ls_wspec(a)), wf64<T>(), SYM_IKX + j, 0, 0.5};

@@ -222,6 +222,9 @@ struct XInvArgs {
     const cpx<double>* tw;
     long nlines = 0;  // lines processed (planes * n for a slab)
     int px = 0;       // row pitch of the inputs in elements (0: nx_in); compile-time kernels only
+    // a second output dx_coef d_x of the first (null: none); compile-time kernels only
+    T* dx[MAX_ARR] = {};
+    double dx_coef[MAX_ARR] = {};
 };
 
 template <typename T>
