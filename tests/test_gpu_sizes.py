@@ -84,6 +84,23 @@ def test_match_run_time_plans(n, precision, monkeypatch):
     _same(b, a, precision)
 
 
+@pytest.mark.parametrize("n,precision", [(16, "fp64"), (48, "fp64"), (48, "mixed"), (96, "fp64"), (192, "mixed")])
+def test_reductions_of_the_z_stage(n, precision, monkeypatch):
+    """Every trial of the line search by a transform, whose z stage sums the
+    spectrum's squares and its products with three others: the chunks of a
+    column's loads have to divide its elements (12 at 3 2^a)."""
+    monkeypatch.setenv("MLQ_LS_TRANSFORM_TRIALS", "1")
+    J = {}
+    for kernels in ("reg", "compile-time"):
+        monkeypatch.setenv("MLQ_PASS_KERNELS", kernels)
+        with mlq.MaxLq(n, 4.0, 1.0, precision=precision, optim_tol=1e-14) as c:
+            c.state_load(c.seed_field(1, 2.0, n / 16))
+            _, _, rec = c.state_iterate(3)
+            J[kernels] = [r["J1"] for r in rec]
+    # FP32 trial values carry noise of 1e-7, which enters J once per iteration
+    assert J["compile-time"] == pytest.approx(J["reg"], rel=1e-9 if precision == "fp64" else 1e-4)
+
+
 @pytest.mark.parametrize("n,precision,variant", [(192, "fp64", 2), (192, "mixed", 1), (192, "mixed", 2),
                                                  (192, "mixed", 8), (384, "mixed", 8)])
 def test_tile_variants_match_default(n, precision, variant, monkeypatch):
