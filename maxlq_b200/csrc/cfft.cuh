@@ -364,7 +364,13 @@ struct YShape {
     // zinv_multi_pair_kernel, PairShape), two resident blocks per SM;
     // 9: the same compiled for three (fewer registers, more warps in flight)
     static constexpr bool PAIR = V == 8 || V == 9;
-    static constexpr int PAIR_MINB = V == 9 ? 3 : 2;
+    // threads per SM that the register budget of V = 8 (9) aims at: 512 (768),
+    // 384 for the 12 elements of 3 2^a; two blocks alone let small blocks take
+    // 255 registers and left 8 warps on an SM (an iteration at 256^3 mixed
+    // 4.73 -> 4.64 ms, 192^3 mixed 2.95 -> 2.87, 128^3 FP64 1.40 -> 1.36)
+    static constexpr int PAIR_THREADS = 4 * (N / (N % 3 == 0 ? 12 : 8));
+    static constexpr int PAIR_MINB = V == 9 ? (PAIR_THREADS < 256 ? 768 / PAIR_THREADS : 3)
+                                            : (PAIR_THREADS < 256 ? (N % 3 == 0 ? 384 : 512) / PAIR_THREADS : 2);
     static constexpr int VB = (CW || MB3) ? 0 : (V >= 3 ? V - 3 : V);
     static constexpr bool THREE = N % 3 == 0;  // 3 2^a: V = 0, 1 (24 elements), 2 (the other tile width) and 8
     static constexpr int EY = CW      ? (N >= 32 ? N / 32 : 1)
@@ -391,7 +397,11 @@ struct YShape {
     static constexpr int CW_SMB = (int)((228 * 1024) / (ZSMEM + 1024));
     static constexpr int CW_RGB = 65536 / (YTHREADS * 96);
     static constexpr int CW_MINB = CW_SMB < CW_RGB ? CW_SMB : CW_RGB;
+    // V = 0 in blocks of less than 256 threads: as many blocks as make 512
+    // threads per SM (384 for 12 FP64 elements), as for the pairs
+    static constexpr int V0_MINB = ((THREE && !F32) ? 384 : 512) / (YTHREADS < 512 ? YTHREADS : 512);
     static constexpr int YMINB = CW ? (CW_MINB < 1 ? 1 : CW_MINB)
+                                    : V == 0 && YTHREADS < 256 ? V0_MINB
                                     : MB3 ? 3 : (TWREG ? 1 : (YTHREADS <= 256 ? 2 : (F32 && EY <= 8 ? 2 : 1)));
     static constexpr bool valid =
         V == 0 || (THREE ? (N >= 192 && ZSMEM <= 200 * 1024 &&
