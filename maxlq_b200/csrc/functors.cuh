@@ -570,8 +570,8 @@ struct FAPow {
     template <typename T>
     __device__ void operator()(const T* in, T* out, double*) const {
         const T s = in[1];
-        const T g = s <= T(0) ? T(0) : sqrt(s);
-        out[0] = in[0] * (k == 1.0 ? g : (T)pow((double)g, k));
+        const double g = s <= T(0) ? 0.0 : sqrt((double)s);  // one rounding, after the power (as FGPow)
+        out[0] = in[0] * (T)(k == 1.0 ? g : pow(g, k));
     }
 };
 
