@@ -143,7 +143,7 @@ class EngineBase {
     // phys(iu..iu+2) = u, phys(idu..idu+8) = grad u, and the fields 63..65,
     // 75..83 hold d and grad d, for the spectra u, d.  tr: after a transport
     // (or Lq norm) at w = u + tau d formed from them, phys 0..2 = w while
-    // idu and 75..83 still hold grad u and grad d.  retract() then records
+    // idu and 75..83 still hold grad u and grad d (q = 4 only).  retract() then records
     // that the state spectrum `next` holds cs * w, and the next gradient
     // program forms u and grad u pointwise instead of transforming them.
     // sac: the transport also left P2(|w|^2), P2(g^2) (physical 18, 19 and

@@ -35,3 +35,31 @@ def test_norm_power_of_a_constant_field_is_rounded_once(q):
             u[0] = float(x)
             want = _power_norm_fp32(x, q, False) ** (2.0 / q)
             assert abs(c.calc_global_Lq_norm(u) - want) <= 1e-14 * want
+
+
+# At q != 4 every gradient transforms the stored state, so an evaluation between two iterations (which overwrites the
+# physical fields of u) changes no bit of what follows.  A run that carried its fields from one retraction to the next
+# would drift from its state instead.
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,q", [(32, 6.0), (32, 8.0), (24, 5.0), (48, 3.0)])
+def test_gradient_of_a_run_is_that_of_its_state(n, q, precision):
+    def run(evaluate):
+        with mlq.MaxLq(n, q, 1.0, precision=precision, optim_tol=0.0) as c:
+            c.state_load(c.seed_field(3, 2.0, n / 12))
+            rec = []
+            for _ in range(6):
+                _, st, r = c.state_iterate(1)
+                rec += r
+                if st:
+                    break
+                if evaluate:
+                    c.state_R()
+            return rec, c.state_store()
+
+    a, ua = run(False)
+    b, ub = run(True)
+    assert len(a) == len(b) >= 4
+    for x, y in zip(a, b):
+        for k in ("alpha", "beta", "norm_grad", "tau", "J1", "n_evals"):
+            assert x[k] == y[k], (x["iter"], k)
+    assert np.array_equal(ua, ub)
