@@ -465,6 +465,7 @@ class Engine : public EngineBase {
     bool lsg_fit_ = false;
     void lsg_setup(const SVec* u, const SVec* d, double tau0 = 0.0);
     void lsg_trial(double tau, double out[3], double* lqq);
+    bool lsg_exact(double tau);
     // ||.||^2 of the power |.|^k of the S and A that the chain reads
     int power_sq(double k);
     // some power of R, the gradient or the norm is a product with A = P2(g^2)
@@ -494,7 +495,7 @@ class Engine : public EngineBase {
     LsPoly ls_c_{};
     bool ls_host_poly_ = true;  // ls_c_ holds this line search's coefficients
     void ls_poly_to_host();     // copies them from the device search's state
-    long long ls_poly_trials_ = 0, ls_fft_trials_ = 0;
+    long long ls_poly_trials_ = 0, ls_fft_trials_ = 0, ls_whole_trials_ = 0;  // whole: R evaluated without a setup
 
     // ---- the line search on the device ----
     // The setup leaves the coefficients in d_ls_ only (ls_dev_), and the
@@ -510,7 +511,7 @@ class Engine : public EngineBase {
     bool ls_transform_trials_ = false;
     bool ls_dev_ = false;
     LsDevState* d_ls_ = nullptr;
-    void* h_ls_ = nullptr;  // pinned: LsParams, LsOut, LsPoly
+    void* h_ls_ = nullptr;  // pinned: LsParams, LsOut (256), LsPoly (512), means of S_a (896)
     struct LsGraph {
         cudaGraphExec_t exec = nullptr;
         long gen = -1;

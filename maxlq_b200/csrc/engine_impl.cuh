@@ -355,6 +355,7 @@ std::string Engine<T>::kernel_config() const {
                     ", \"graph_replays\": " + std::to_string(graph_launches_) +
                     ", \"line_search_trials_polynomial\": " + std::to_string(ls_poly_trials_) +
                     ", \"line_search_trials_transform\": " + std::to_string(ls_fft_trials_) +
+                    ", \"line_search_trials_whole\": " + std::to_string(ls_whole_trials_) +
                     ", \"line_searches_on_device\": " + std::to_string(ls_dev_searches_) +
                     ", \"line_search_device_passes\": " + std::to_string(ls_dev_loops_) +
                     ", \"device_bytes_peak\": " + std::to_string(bytes_peak) +
@@ -3065,6 +3066,26 @@ void Engine<T>::lsg_setup(const SVec* u, const SVec* d, double tau0) {
     lsg_ud_ = lf.ud;
     if (lsg_poly_ok()) lsg_poly_setup();
     ls_interval_dev(tau0);
+    // the means of S_a (k = 0), read by lsg_exact with the intervals
+    for (int a = 0; a < 3; ++a)
+        MLQ_CUDA(cudaMemcpyAsync((cpx<T>*)((char*)h_ls_ + 896) + a, wspec(ls_wspec(a)), sizeof(cpx<T>),
+                                 cudaMemcpyDeviceToHost, stream));
+}
+
+// Whether trials from the coefficient fields are as exact as fields of
+// phi = u + tau d formed anew.  Relative to |phi|^2, |phi|^2 from its
+// coefficients carries the rounding of (|u| + |tau d|)^2, and from phi twice that
+// of (|u| + |tau d|) |phi|: the coefficients are the better ones while
+// |u| + |tau d| <= 2 |phi|, in L2 norms here.  For orthogonal u and d, as of a CG
+// search, the left side is at most 1.42 |phi|; directions that undo u fail it,
+// and their trials evaluate R whole.
+template <typename T>
+bool Engine<T>::lsg_exact(double tau) {
+    ls_poly_to_host();
+    const cpx<T>* m = (const cpx<T>*)((const char*)h_ls_ + 896);
+    const double s0 = m[0].x, s1 = m[1].x, s2 = m[2].x;
+    const double sum = std::sqrt(std::max(s0, 0.0)) + std::fabs(tau) * std::sqrt(std::max(s2, 0.0));
+    return sum * sum <= 4.0 * (s0 + tau * (s1 + tau * s2));
 }
 
 // The Parseval products of two polynomial spectra, by power of tau: one pass
@@ -3230,7 +3251,6 @@ void Engine<T>::lsg_trial(double tau, double out[3], double* lqq) {
         out[2] = R3;
     };
     if (free_tau && lsg_poly_ok()) {
-        ++ls_poly_trials_;
         const int nc = q == 8.0 ? 5 : 3;
         if (nc == 3) {
             FLSS32 f;
@@ -3247,14 +3267,21 @@ void Engine<T>::lsg_trial(double tau, double out[3], double* lqq) {
             std::copy(h_results + RNRM, h_results + RNRM + 9, lsg_nrm_);
             lsg_poly_fetched_ = true;
         }
-        auto poly = [&](const double* c, int m) {
+        auto poly = [&](const double* c, int m, bool abs = false) {
             double v = 0.0;
-            for (int k = m - 1; k >= 0; --k) v = v * tau + c[k];
+            for (int k = m - 1; k >= 0; --k) v = abs ? v * std::fabs(tau) + std::fabs(c[k]) : v * tau + c[k];
             return v;
         };
-        result(poly(lsg_i1_, nc + 4), poly(lsg_i2_, nc + 4), poly(lsg_i3_, nc + 5));
-        if (lqq) *lqq = nc == 3 ? h_results[130] : poly(lsg_nrm_, 9);
-        return;
+        // |phi|^q from phi carries q times the rounding of phi, the sum of a
+        // polynomial that of its terms: where they cancel by more than q in
+        // one of the positive integrals, the trial below takes over
+        auto exact = [&](const double* c, int m) { return poly(c, m, true) <= q * poly(c, m); };
+        if (exact(lsg_i1_, nc + 4) && (nc == 3 || exact(lsg_nrm_, 9))) {
+            ++ls_poly_trials_;
+            result(poly(lsg_i1_, nc + 4), poly(lsg_i2_, nc + 4), poly(lsg_i3_, nc + 5));
+            if (lqq) *lqq = nc == 3 ? h_results[130] : poly(lsg_nrm_, 9);
+            return;
+        }
     }
     if (free_tau) {
         // S(tau) >= 0 at every point: A = P2(max(S, 0)) = S

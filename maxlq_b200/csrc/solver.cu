@@ -111,10 +111,13 @@ class Solver : public SolverBase {
         Trial t;
         if (ls_ready)
             e.ls_trial(tau, t.R, &t.lqq);
-        else if (lsg_ready)
+        else if (lsg_ready && e.lsg_exact(tau))
             e.lsg_trial(tau, t.R, &t.lqq);
-        else
+        else {
+            lsg_ready = false;  // the evaluation overwrites the coefficient fields
+            ++e.ls_whole_trials_;
             e.R_eval(base, dir, tau, t.R, &t.lqq);
+        }
         trials[tau] = t;
         return t;
     }

@@ -63,3 +63,40 @@ def test_gradient_of_a_run_is_that_of_its_state(n, q, precision):
         for k in ("alpha", "beta", "norm_grad", "tau", "J1", "n_evals"):
             assert x[k] == y[k], (x["iter"], k)
     assert np.array_equal(ua, ub)
+
+
+# A direction that undoes the base field: phi + tau d near tau = T is 64 times smaller than phi.  Sums of coefficient
+# fields lose 64^2 there, polynomials of degree q 64^q; such trials evaluate R whole.  Those carry some q 64 roundings,
+# 1e-13 of J at most, which moves Brent's minimum by some sqrt(1e-13) = 3e-7 of the bracket; the bound leaves a
+# factor of 300.
+@pytest.mark.parametrize("n,q", [(32, 6.0), (32, 8.0), (24, 8.0)])
+def test_search_along_a_direction_that_undoes_the_field(n, q, monkeypatch):
+    def search(reuse):
+        monkeypatch.setenv("MLQ_REUSE", reuse)
+        with mlq.MaxLq(n, q, 1.0) as c:
+            v = c.rescaleLqNorm(c.seed_field(2, 2.0, n / 12))
+            w = c.divAvg_free(c.HilbertGradient(c.GradL2ForLq(v), 1.5 - 1.0 / q))
+            w *= np.sqrt((v * v).sum() / (w * w).sum())
+            tb, flag = c.mnbrak(v, w, 0.0, 1.0)
+            assert flag == 0
+            T = 64.0
+            return tb, c.brent(v - T * w, w, T + tb) - T, c.kernel_config()
+
+    tb, x0, _ = search("0")
+    _, x1, cfg = search("1")
+    assert tb[0] < x0 < tb[1]
+    assert abs(x1 - x0) <= 1e-4 * (tb[1] - tb[0])
+    assert cfg["line_search_trials_whole"] > 0
+
+
+# and a search of a run, whose directions are tangent to the constraint, needs none of them
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,q", [(32, 3.0), (32, 5.0), (48, 6.0), (32, 8.0)])
+def test_searches_of_a_run_use_the_coefficient_fields(n, q, precision):
+    with mlq.MaxLq(n, q, 1.0, precision=precision, optim_tol=0.0) as c:
+        c.state_load(c.seed_field(3, 2.0, n / 12))
+        c.state_iterate(6)
+        cfg = c.kernel_config()
+    assert cfg["line_search_trials_whole"] == 0
+    if q in (6.0, 8.0):
+        assert cfg["line_search_trials_polynomial"] > 0
