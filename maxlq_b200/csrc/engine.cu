@@ -61,6 +61,8 @@ EngineBase::EngineBase(const mlq_params& p) : P(p) {
     if (const char* e = std::getenv("MLQ_PDL")) pdl_on_ = std::string(e) != "0";
     pdl_ = pdl_on_;
     if (const char* e = std::getenv("MLQ_REUSE")) reuse_on_ = std::string(e) != "0";
+    if (const char* e = std::getenv("MLQ_INJECT"))
+        if (const char* k = std::strstr(e, "transport-nan=")) inject_nan_ = std::atoi(k + 14);
     if (const char* e = std::getenv("MLQ_ZMULTI")) multi_zinv_ = std::string(e) != "0";
 }
 
@@ -149,6 +151,10 @@ void EngineBase::fetch_results() {
         MLQ_CUDA(cudaMemsetAsync(d_results + NAN_SLOT, 0, sizeof(double), stream));
         MLQ_CUDA(cudaStreamSynchronize(stream));
         h_results[NAN_SLOT] = 0.0;
+        // what is remembered of the fields may tell of a retraction that the
+        // flag kept from writing
+        pm_ = PhysMemo{};
+        pu_of_ = ws_of_ = nullptr;
         throw CudaError("NaN or Inf in a field entering a forward transform", MLQ_ERR_NAN);
     }
 }

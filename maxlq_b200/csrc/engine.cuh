@@ -215,6 +215,9 @@ class EngineBase {
     // line search's coefficients, W as half-gradients of |phi|^2); MLQ_REUSE=0
     // runs every program in its plain transform sequence instead
     bool reuse_on_ = true;
+    // failures made on the host, for tests (MLQ_INJECT): "transport-nan=k" raises
+    // the NaN flag in the k-th transport
+    int inject_nan_ = 0;
     // single-source z inverse launches grouped by source (one load per
     // column for a field and its derivatives); MLQ_ZMULTI=0 turns it off
     bool multi_zinv_ = true;

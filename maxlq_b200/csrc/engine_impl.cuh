@@ -2334,6 +2334,10 @@ int Engine<T>::transport_async(const SVec* u, const SVec* d, double tau, const S
     SpecDotPair pr[6];
     for (int i = 0; i < nxi; ++i) pr[i] = SpecDotPair{cbuf, xi[i], 0};
     dots_async(pr, nxi);
+    if (inject_nan_ > 0 && --inject_nan_ == 0) {
+        static const double one = 1.0;
+        MLQ_CUDA(cudaMemcpyAsync(d_results + NAN_SLOT, &one, sizeof(one), cudaMemcpyHostToDevice, stream));
+    }
     return slot;
 }
 

@@ -1,0 +1,40 @@
+"""What a context does after a failure inside an iteration.  The failures are made on the host (MLQ_INJECT)."""
+import numpy as np
+import pytest
+
+import maxlq_b200 as mlq
+
+pytestmark = pytest.mark.gpu
+
+
+
+# A NaN met in the transport leaves the state as it was, and the next iteration is the one that failed, done again.  Its
+# gradient transforms the state where the run that did not fail forms u from the retraction: 1e-13 apart, which Brent's
+# flat minimum turns into 1e-7 of the step and the cancellation of deltaJ into 1e-9 of J.
+@pytest.mark.parametrize("n,q", [(64, 4.0), (48, 4.0), (32, 6.0)])
+def test_iteration_after_a_nan_in_the_transport(n, q, monkeypatch):
+    def start():
+        c = mlq.MaxLq(n, q, 1.0, optim_tol=0.0)
+        c.state_load(c.seed_field(1, 2.0, n / 12))
+        return c
+
+    with start() as c:
+        c.state_iterate(1)
+        u1 = c.state_store()
+        _, st, good = c.state_iterate(1)
+        assert st == 0
+        u2 = c.state_store()
+    monkeypatch.setenv("MLQ_INJECT", "transport-nan=2")
+    with start() as c:
+        c.state_iterate(1)
+        with pytest.raises(mlq.MlqError) as e:
+            c.state_iterate(1)
+        assert e.value.status == mlq.MLQ_ERR_NAN
+        assert np.array_equal(c.state_store(), u1)
+        _, st, again = c.state_iterate(1)
+        assert st == 0
+        a, g = again[0], good[0]
+        for k in ("alpha", "beta", "norm_grad", "norm_d1", "J0", "J1"):
+            assert abs(a[k] - g[k]) <= 1e-9 * abs(g[k]), k
+        assert abs(a["tau"] - g["tau"]) <= 1e-6 * g["tau"]
+        assert np.abs(c.state_store() - u2).max() <= 1e-6 * np.abs(u2).max()
