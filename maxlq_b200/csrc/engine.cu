@@ -61,8 +61,10 @@ EngineBase::EngineBase(const mlq_params& p) : P(p) {
     if (const char* e = std::getenv("MLQ_PDL")) pdl_on_ = std::string(e) != "0";
     pdl_ = pdl_on_;
     if (const char* e = std::getenv("MLQ_REUSE")) reuse_on_ = std::string(e) != "0";
-    if (const char* e = std::getenv("MLQ_INJECT"))
+    if (const char* e = std::getenv("MLQ_INJECT")) {
         if (const char* k = std::strstr(e, "transport-nan=")) inject_nan_ = std::atoi(k + 14);
+        inject_ls_graph_ = std::strstr(e, "ls-graph") != nullptr;
+    }
     if (const char* e = std::getenv("MLQ_ZMULTI")) multi_zinv_ = std::string(e) != "0";
 }
 

@@ -216,8 +216,10 @@ class EngineBase {
     // runs every program in its plain transform sequence instead
     bool reuse_on_ = true;
     // failures made on the host, for tests (MLQ_INJECT): "transport-nan=k" raises
-    // the NaN flag in the k-th transport
+    // the NaN flag in the k-th transport, "ls-graph" fails the build of the device
+    // search's graph
     int inject_nan_ = 0;
+    bool inject_ls_graph_ = false;
     // single-source z inverse launches grouped by source (one load per
     // column for a field and its derivatives); MLQ_ZMULTI=0 turns it off
     bool multi_zinv_ = true;

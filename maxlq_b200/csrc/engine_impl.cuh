@@ -2819,6 +2819,7 @@ static cudaGraph_t add_conditional(cudaGraph_t g, cudaGraphNode_t dep, cudaGraph
 // after LS_MAX_LOOPS passes, so the loop is bounded whatever the kernels see.
 template <typename T>
 bool Engine<T>::ls_graph_build(LsGraph& g, int key) {
+    if (inject_ls_graph_) return false;
     if (g.exec) cudaGraphExecDestroy(g.exec);
     g.exec = nullptr;
     const int grid = grid_for(n3, RED_THREADS, 148 * 4);
@@ -2924,6 +2925,7 @@ int Engine<T>::ls_device_search(double B, double tA0, double tB0, LsOut* out) {
             }
         if (!ls_graph_build(*g, key)) {
             lsg_failed_ = true;
+            fetch_results();  // the setup left its sums, and the update's, to this search's fetch
             return 1;
         }
     }

@@ -38,3 +38,25 @@ def test_iteration_after_a_nan_in_the_transport(n, q, monkeypatch):
             assert abs(a[k] - g[k]) <= 1e-9 * abs(g[k]), k
         assert abs(a["tau"] - g["tau"]) <= 1e-6 * g["tau"]
         assert np.abs(c.state_store() - u2).max() <= 1e-6 * np.abs(u2).max()
+
+
+# Where the device search's graph cannot be built the search runs on the host, and the iteration's record holds this
+# update's scalars.  The field is smooth enough that every trial is a polynomial, so that no trial's fetch brings them.
+@pytest.mark.parametrize("iters", [1, 3])
+def test_record_of_a_search_without_its_graph(iters, monkeypatch):
+    def run():
+        with mlq.MaxLq(64, 4.0, 1.0, optim_tol=0.0) as c:
+            u = c.seed_field(1, 2.0, 0.7)
+            c.state_load(u)
+            _, st, rec = c.state_iterate(iters)
+            assert st == 0
+            return rec, c.kernel_config()
+
+    dev, cfg = run()
+    assert cfg["line_searches_on_device"] == iters and cfg["line_search_trials_transform"] == 0
+    monkeypatch.setenv("MLQ_INJECT", "ls-graph")
+    host, cfg = run()
+    assert cfg["line_searches_on_device"] == 0 and cfg["line_search_trials_transform"] == 0
+    for a, b in zip(host, dev):
+        for k in ("alpha", "beta", "norm_grad", "norm_td0", "norm_d1", "tau", "J1"):
+            assert abs(a[k] - b[k]) <= 1e-9 * abs(b[k]), (b["iter"], k)
