@@ -114,6 +114,7 @@ namespace {
 template <class Fn>
 int guard(mlq_ctx* c, Fn fn) {
     if (!c) return MLQ_ERR_BADARG;
+    const EngineBase::InUse use(c->solver ? &c->solver->eng() : nullptr);
     try {
         fn();
         c->err.clear();

@@ -63,6 +63,7 @@ EngineBase::EngineBase(const mlq_params& p) : P(p) {
     if (const char* e = std::getenv("MLQ_REUSE")) reuse_on_ = std::string(e) != "0";
     if (const char* e = std::getenv("MLQ_INJECT")) {
         if (const char* k = std::strstr(e, "transport-nan=")) inject_nan_ = std::atoi(k + 14);
+        if (const char* k = std::strstr(e, "search-oom=")) inject_oom_ = std::atoi(k + 11);
         inject_ls_graph_ = std::strstr(e, "ls-graph") != nullptr;
     }
     if (const char* e = std::getenv("MLQ_ZMULTI")) multi_zinv_ = std::string(e) != "0";
@@ -103,9 +104,47 @@ FftPlan EngineBase::plan(int L) const {
     return p;
 }
 
+namespace {
+struct Contexts {
+    std::mutex mu;
+    std::vector<EngineBase*> all;
+};
+Contexts& contexts() {
+    static Contexts c;
+    return c;
+}
+}  // namespace
+
+void EngineBase::contexts_add(EngineBase* e) {
+    std::lock_guard<std::mutex> l(contexts().mu);
+    contexts().all.push_back(e);
+}
+void EngineBase::contexts_remove(EngineBase* e) {
+    std::lock_guard<std::mutex> l(contexts().mu);
+    auto& a = contexts().all;
+    a.erase(std::remove(a.begin(), a.end(), e), a.end());
+}
+EngineBase::InUse::InUse(EngineBase* e_) : e(e_) {
+    std::lock_guard<std::mutex> l(contexts().mu);
+    if (e) ++e->in_use_;
+}
+EngineBase::InUse::~InUse() {
+    std::lock_guard<std::mutex> l(contexts().mu);
+    if (e) --e->in_use_;
+}
+
 void* EngineBase::dev_alloc(size_t b) {
     void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, b);
+    const bool inject = in_search_ && inject_oom_ > 0 && --inject_oom_ == 0;
+    cudaError_t e = inject ? cudaErrorMemoryAllocation : cudaMalloc(&p, b);
+    if (e == cudaErrorMemoryAllocation && !inject) {
+        cudaGetLastError();
+        // a context enters a call under the same lock, so none does meanwhile
+        std::lock_guard<std::mutex> l(contexts().mu);
+        for (EngineBase* c : contexts().all)
+            if (c->in_use_ == 0 && c->P.device == P.device) c->give_back();
+        e = cudaMalloc(&p, b);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         throw CudaError("cudaMalloc of " + std::to_string(b) + " bytes failed: " + cudaGetErrorString(e),
@@ -133,6 +172,8 @@ SVec* EngineBase::alloc_state() { return dev_alloc(3 * spec_ncomp() * sv_elem())
 void EngineBase::ensure_partials(long cnt) {
     if (cnt <= partials_cap) return;
     if (d_partials) free_dev(d_partials);
+    d_partials = nullptr;  // stays so if the allocation throws
+    partials_cap = 0;
     d_partials = (double*)dev_alloc(cnt * sizeof(double));
     partials_cap = cnt;
 }

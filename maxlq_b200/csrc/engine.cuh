@@ -217,9 +217,21 @@ class EngineBase {
     bool reuse_on_ = true;
     // failures made on the host, for tests (MLQ_INJECT): "transport-nan=k" raises
     // the NaN flag in the k-th transport, "ls-graph" fails the build of the device
-    // search's graph
-    int inject_nan_ = 0;
+    // search's graph, "search-oom=k" the k-th allocation inside searches
+    int inject_nan_ = 0, inject_oom_ = 0;
     bool inject_ls_graph_ = false;
+    bool in_search_ = false;
+    // Contexts of the process.  Where an allocation fails, contexts that are in
+    // no call give back what they can do without.
+    static void contexts_add(EngineBase* e);
+    static void contexts_remove(EngineBase* e);
+    struct InUse {  // the context of e is in a call
+        EngineBase* e;
+        explicit InUse(EngineBase* e_);
+        ~InUse();
+    };
+    int in_use_ = 0;
+    virtual void give_back() {}
     // single-source z inverse launches grouped by source (one load per
     // column for a field and its derivatives); MLQ_ZMULTI=0 turns it off
     bool multi_zinv_ = true;
@@ -467,7 +479,13 @@ class Engine : public EngineBase {
     // are not.  Resident mode only; MLQ_REUSE=0 evaluates R whole per trial.
     bool lsg_ok() const { return !ls_ok() && !slab_ && reuse_on_; }
     bool lsg_fits();
-    bool lsg_fit_ = false;
+    void lsg_release();
+    void lsg_give_up();
+    void lsg_retry() { lsg_refused_ = false; }
+    void give_back() override { lsg_release(); }
+    void* lsg_block_ = nullptr;
+    std::vector<int> lsg_slices_;  // physical fields in the block
+    bool lsg_refused_ = false;
     void lsg_setup(const SVec* u, const SVec* d, double tau0 = 0.0);
     void lsg_trial(double tau, double out[3], double* lqq);
     bool lsg_exact(double tau);

@@ -1427,7 +1427,7 @@ template <typename T>
 void Engine<T>::release_io_buffers() {
     pu_of_ = nullptr;
     pm_ = PhysMemo{};
-    lsg_fit_ = false;
+    lsg_release();
     for (auto* v : {&phys_}) {
         for (auto*& p : *v) {
             if (p) free_dev(p);
@@ -3034,25 +3034,67 @@ void Engine<T>::ls_trial(double tau, double out[3], double* lqq) {
 // the copy rate) and a CG iteration 138 instead of 383; two iterations at
 // 256^3 q = 6 FP64 take 83 instead of 187 ms with their transfers.
 
-// The fields of the setup and the trials fit next to what is allocated.
-// Asked until they do, since cudaMemGetInfo stalls for up to 100 ms at times;
-// the first search allocates them.
+// The fields of the setup and the trials, in one block: it fits whole or not at
+// all, and costs one allocation (49 of 2 MB take 15 ms, one of 98 MB 0.4).  The
+// first search of a context takes it, up to 0.8 of what is free; where it does
+// not fit, trials evaluate R whole until lsg_retry.  Other contexts that run out
+// of memory may have it back while this one is in no call (give_back).
 template <typename T>
 bool Engine<T>::lsg_fits() {
-    if (lsg_fit_) return true;
-    long need = 8;  // transform buffers and partials
+    if (lsg_block_) return true;
+    if (lsg_refused_) return false;
+    std::vector<int> need;
     for (int i = LU; i < LEND; ++i) {
         const bool used = i < LP + 3 ? (!use_e_u || i < LV || i >= LP)
                           : i < LTS  ? false
                           : i < LW   ? true
                           : i < LC   ? use_e_u
                                      : lsg_poly_ok() && P.q == 8.0;
-        if (used && ((int)phys_.size() <= i || !phys_[i])) ++need;
+        if (used && ((int)phys_.size() <= i || !phys_[i])) need.push_back(i);
     }
+    const size_t each = ((size_t)n3 * sizeof(T) + 255) / 256 * 256;
     size_t fr = 0, tot = 0;
     MLQ_CUDA(cudaMemGetInfo(&fr, &tot));
-    lsg_fit_ = (double)need * (double)n3 * sizeof(T) < 0.8 * (double)fr;
-    return lsg_fit_;
+    lsg_refused_ = true;
+    // 8 more: transform buffers and partials
+    if ((double)(need.size() + 8) * (double)each >= 0.8 * (double)fr) return false;
+    try {
+        lsg_block_ = dev_alloc(std::max<size_t>(1, need.size()) * each);
+    } catch (const CudaError& x) {
+        if (x.status != MLQ_ERR_OOM) throw;
+        return false;
+    }
+    lsg_refused_ = false;
+    if ((int)phys_.size() < LEND) phys_.resize(LEND, nullptr);
+    for (size_t k = 0; k < need.size(); ++k) phys_[need[k]] = (T*)((char*)lsg_block_ + k * each);
+    lsg_slices_ = need;
+    return true;
+}
+
+// The block and the search's work spectra back to the device.
+template <typename T>
+void Engine<T>::lsg_release() {
+    if (!lsg_block_) return;
+    MLQ_CUDA(cudaStreamSynchronize(stream));
+    pm_ = PhysMemo{};
+    for (int i : lsg_slices_) phys_[i] = nullptr;
+    lsg_slices_.clear();
+    free_dev(lsg_block_);
+    lsg_block_ = nullptr;
+    for (int i = 0; i < (int)ws_.size(); ++i)
+        if (ws_[i] && ((i >= WLS && i < WLS + 3) || (i >= WLQ && i < WLQ + 3) || (i >= WLC && i < WLU + 4))) {
+            free_dev(ws_[i]);
+            ws_[i] = nullptr;
+        }
+}
+
+// A search that ran out of memory: its fields back, and whole evaluations for
+// the rest of the run.
+template <typename T>
+void Engine<T>::lsg_give_up() {
+    cudaGetLastError();
+    lsg_release();
+    lsg_refused_ = true;
 }
 
 template <typename T>

@@ -63,7 +63,9 @@ class Solver : public SolverBase {
         c = e.alloc_state();
         tmp = e.alloc_state();
         tmp2 = nullptr;
+        EngineBase::contexts_add(&e);
     }
+    ~Solver() override { EngineBase::contexts_remove(&e); }
     EngineBase& eng() override { return e; }
     long nc() const { return e.spec_ncomp(); }
     double q() const { return e.P.q; }
@@ -100,9 +102,29 @@ class Solver : public SolverBase {
         if (e.ls_ok() && dir && e.ls_fits()) {
             e.ls_setup(base, dir, tau_near);
             ls_ready = true;
-        } else if (e.lsg_ok() && dir && e.lsg_fits()) {
-            e.lsg_setup(base, dir, tau_near);
-            lsg_ready = true;
+        } else if (e.lsg_ok() && dir) {
+            lsg_ready = in_search([&] {
+                if (!e.lsg_fits()) return false;
+                e.lsg_setup(base, dir, tau_near);
+                return true;
+            });
+        }
+    }
+    // false where f returned false or ran out of memory (the coefficient fields
+    // are given back then)
+    template <class Fn>
+    bool in_search(Fn&& f) {
+        struct Flag {
+            bool& b;
+            explicit Flag(bool& b_) : b(b_) { b = true; }
+            ~Flag() { b = false; }
+        } flag(e.in_search_);
+        try {
+            return f();
+        } catch (const CudaError& x) {
+            if (x.status != MLQ_ERR_OOM) throw;
+            e.lsg_give_up();
+            return false;
         }
     }
     Trial trial(const SVec* base, const SVec* dir, double tau) {
@@ -111,9 +133,10 @@ class Solver : public SolverBase {
         Trial t;
         if (ls_ready)
             e.ls_trial(tau, t.R, &t.lqq);
-        else if (lsg_ready && e.lsg_exact(tau))
-            e.lsg_trial(tau, t.R, &t.lqq);
-        else {
+        else if (!(lsg_ready && e.lsg_exact(tau) && in_search([&] {
+                     e.lsg_trial(tau, t.R, &t.lqq);
+                     return true;
+                 }))) {
             lsg_ready = false;  // the evaluation overwrites the coefficient fields
             ++e.ls_whole_trials_;
             e.R_eval(base, dir, tau, t.R, &t.lqq);
@@ -185,6 +208,7 @@ class Solver : public SolverBase {
         avg_imp = 1.0;
         while_flag = 0;
         started = true;
+        e.lsg_retry();
     }
 
     // one iteration of optimization.f90:136-446; returns status
