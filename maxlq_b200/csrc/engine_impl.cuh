@@ -366,7 +366,8 @@ std::string Engine<T>::kernel_config() const {
 // Autotuner: time every valid y/z tile-shape variant of each pass kind on
 // scratch buffers of the state band (three arrays, as the programs launch
 // them) and keep the fastest.  Runs once per engine, before the programs
-// allocate their buffers.  MLQ_AUTOTUNE=0 keeps variant 0 everywhere.
+// allocate their buffers; 3 2^a has a rule instead.  MLQ_AUTOTUNE=0 keeps
+// variant 0 everywhere.
 template <typename T>
 void Engine<T>::tune_yz() {
     tune_report_.clear();
@@ -418,6 +419,19 @@ void Engine<T>::tune_yz() {
         if (ok)
             for (int k = 0; k < YV_KINDS; ++k) yvar_[k] = v;
         tune_report_ = std::string("fixed by MLQ_YZ_VARIANT=") + e;
+        return;
+    }
+    // 3 2^a: by rule, as timing the few variants makes mlq_init at 192^3 mixed 14
+    // instead of 5 ms (45 at 384^3) for what always comes out the same: in FP32 the
+    // column pairs (y 31.8 and 33.6 us at 192^3 and 225 and 232 at 384^3 against
+    // 37.8, 37.6 and 289, 282 of variant 0, z inverse 27.8 and 201 against 29.4 and
+    // 269, round trip 39.4 and 299 against 42.4 and 336, z forward 38.5 and 249
+    // against 37.6 and 251); in FP64 variant 0 (variant 2: 3 to 26 % slower).
+    if (n % 3 == 0) {
+        int v = 0;
+        dispatch_n(n, [&](auto nc) { v = YShape<decltype(nc)::value, T, 8>::valid ? 8 : 0; });
+        for (int k = 0; k < YV_KINDS; ++k) yvar_[k] = v;
+        tune_report_ = "v" + std::to_string(v) + " by rule";
         return;
     }
     const Band b = b2;
