@@ -53,7 +53,6 @@ EngineBase::EngineBase(const mlq_params& p) : P(p) {
     MLQ_CUDA(cudaMemcpyAsync(d_tw, pool.data(), pool.size() * sizeof(cpx<double>), cudaMemcpyHostToDevice, stream));
     MLQ_CUDA(cudaStreamSynchronize(stream));
     d_results = (double*)dev_alloc(NRES * sizeof(double));
-    MLQ_CUDA(cudaMallocHost((void**)&h_results, NRES * sizeof(double)));
     MLQ_CUDA(cudaMemsetAsync(d_results, 0, NRES * sizeof(double), stream));
     MLQ_CUDA(cudaStreamSynchronize(stream));
     ensure_partials(1 << 20);
@@ -73,7 +72,6 @@ EngineBase::~EngineBase() {
     for (auto& kv : graphs_)
         if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
     for (auto& a : allocs_) cudaFree(a.first);
-    if (h_results) cudaFreeHost(h_results);
     if (stream) cudaStreamDestroy(stream);
 }
 

@@ -2601,9 +2601,11 @@ void Engine<T>::ls_qg_fields(const LsFields& lf, bool g_phys) {
 // the line search's state on the device, and its pinned host side
 template <typename T>
 void Engine<T>::ls_dev_alloc() {
-    if (d_ls_) return;
-    d_ls_ = (LsDevState*)dev_alloc(sizeof(LsDevState));
-    MLQ_CUDA(cudaMallocHost(&h_ls_, 1024));
+    if (!d_ls_) d_ls_ = (LsDevState*)dev_alloc(sizeof(LsDevState));
+    if (h_ls_) return;
+    MLQ_CUDA(cudaMallocHost(&h_ls_, 1024 + NRES * sizeof(double)));
+    h_results = (double*)((char*)h_ls_ + 1024);
+    std::copy(h_results_, h_results_ + NRES, h_results);
 }
 
 // clamp-free intervals of S(tau) and the polynomial coefficients, left on
