@@ -3130,7 +3130,7 @@ void Engine<T>::lsg_setup(const SVec* u, const SVec* d, double tau0) {
     lsg_ud_ = lf.ud;
     if (lsg_poly_ok()) lsg_poly_setup();
     ls_interval_dev(tau0);
-    // the means of S_a (k = 0), read by lsg_exact with the intervals
+    // the means of S_a (k = 0), read with the intervals (lsg_exact)
     for (int a = 0; a < 3; ++a)
         MLQ_CUDA(cudaMemcpyAsync((cpx<T>*)((char*)h_ls_ + 896) + a, wspec(ls_wspec(a)), sizeof(cpx<T>),
                                  cudaMemcpyDeviceToHost, stream));
@@ -3140,16 +3140,18 @@ void Engine<T>::lsg_setup(const SVec* u, const SVec* d, double tau0) {
 // phi = u + tau d formed anew.  Relative to |phi|^2, |phi|^2 from its
 // coefficients carries the rounding of (|u| + |tau d|)^2, and from phi twice that
 // of (|u| + |tau d|) |phi|: the coefficients are the better ones while
-// |u| + |tau d| <= 2 |phi|, in L2 norms here.  For orthogonal u and d, as of a CG
-// search, the left side is at most 1.42 |phi|; directions that undo u fail it,
-// and their trials evaluate R whole.
+// |u| + |tau d| <= 2 |phi|, in L2 norms here.  On a side of tau that holds for
+// every tau where u and tau d have a cosine of -1/2 or more.  The directions of
+// runs (q = 3 to 12) had -0.36 to 0.67; full gradients, which undo u, -0.98 to
+// -0.59, with polynomial sums of terms up to 1e4 times their value.  All trials of
+// such a search evaluate R whole: values formed both ways differ by their
+// rounding, too much for a bracket around a small step in FP32.
 template <typename T>
 bool Engine<T>::lsg_exact(double tau) {
     ls_poly_to_host();
     const cpx<T>* m = (const cpx<T>*)((const char*)h_ls_ + 896);
-    const double s0 = m[0].x, s1 = m[1].x, s2 = m[2].x;
-    const double sum = std::sqrt(std::max(s0, 0.0)) + std::fabs(tau) * std::sqrt(std::max(s2, 0.0));
-    return sum * sum <= 4.0 * (s0 + tau * (s1 + tau * s2));
+    const double s0 = m[0].x, s1 = m[1].x, s2 = m[2].x;  // s1 = 2 <u, d>
+    return (tau < 0.0 ? -s1 : s1) >= -std::sqrt(s0 * s2);
 }
 
 // The Parseval products of two polynomial spectra, by power of tau: one pass

@@ -100,3 +100,23 @@ def test_searches_of_a_run_use_the_coefficient_fields(n, q, precision):
     assert cfg["line_search_trials_whole"] == 0
     if q in (6.0, 8.0):
         assert cfg["line_search_trials_polynomial"] > 0
+
+
+# All trials of one search are formed one way: mnbrak along the full gradient (which undoes the field) brackets as with
+# whole evaluations, also where steps are so small that J changes by the rounding of FP32.
+@pytest.mark.parametrize("n,q", [(64, 5.0), (64, 3.0), (64, 8.0)])
+def test_bracket_along_the_full_gradient_in_mixed_precision(n, q, monkeypatch):
+    def search(reuse):
+        monkeypatch.setenv("MLQ_REUSE", reuse)
+        with mlq.MaxLq(n, q, 1.0, precision="mixed") as c:
+            u = c.rescaleLqNorm(c.seed_field(0, 2.0, n / 12))
+            d = c.divAvg_free(c.HilbertGradient(c.GradL2ForLq(u), 1.5 - 1.0 / q))
+            d *= np.sqrt((u * u).sum() / (d * d).sum())
+            tb, flag = c.mnbrak(u, d, 0.0, 1.0)
+            return tb, flag, c.kernel_config()
+
+    _, f0, c0 = search("0")
+    _, f1, c1 = search("1")
+    assert f0 == f1
+    n0, n1 = c0["line_search_trials_whole"], c1["line_search_trials_whole"]
+    assert n1 > 0 and c1["line_search_trials_polynomial"] == c1["line_search_trials_transform"] == 0
