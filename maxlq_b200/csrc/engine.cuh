@@ -24,7 +24,7 @@ namespace mlq {
 
 // launchers of the device line search's kernels (lsdev.cu)
 void ls_launch_coef(LsDevState* s, const double* results, const double* partials, int nblocks, const LsAnchorSet& an,
-                    cudaStream_t st);
+                    bool pdl, cudaStream_t st);
 void ls_launch_ctrl(LsDevState* s, const double* r, int direct, cudaGraphConditionalHandle h_loop,
                     cudaGraphConditionalHandle h_next, cudaStream_t st);
 

@@ -2620,7 +2620,7 @@ void Engine<T>::ls_interval_dev(double tau0) {
     launch_k(ls_interval_kernel<T>, grid, RED_THREADS, 0, phys(ls_phys(0)), phys(ls_phys(1)), phys(ls_phys(2)), n3,
                                                             an, d_partials);
     launched("ls_interval", 3.0 * n3 * sizeof(T), ev);
-    ls_launch_coef(d_ls_, d_results, d_partials, grid, an, stream);
+    ls_launch_coef(d_ls_, d_results, d_partials, grid, an, pdl_, stream);
     launched();
     ls_host_poly_ = false;
 }

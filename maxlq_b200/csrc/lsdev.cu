@@ -218,8 +218,8 @@ __global__ void ls_ctrl_kernel(LsDevState* s, const double* __restrict__ sums, i
 }
 
 void ls_launch_coef(LsDevState* s, const double* results, const double* partials, int nblocks, const LsAnchorSet& an,
-                    cudaStream_t st) {
-    MLQ_CUDA(launch_pdl(true, ls_coef_kernel, 1, LS_COEF_THREADS, 0, st, s, results, partials, nblocks, an));
+                    bool pdl, cudaStream_t st) {
+    MLQ_CUDA(launch_pdl(pdl, ls_coef_kernel, 1, LS_COEF_THREADS, 0, st, s, results, partials, nblocks, an));
 }
 void ls_launch_ctrl(LsDevState* s, const double* r, int direct, cudaGraphConditionalHandle h_loop,
                     cudaGraphConditionalHandle h_next, cudaStream_t st) {
