@@ -3352,9 +3352,9 @@ void Engine<T>::lsg_trial(double tau, double out[3], double* lqq) {
             return;
         }
     }
+    ++ls_fft_trials_;
     if (free_tau) {
         // S(tau) >= 0 at every point: A = P2(max(S, 0)) = S
-        ++ls_poly_trials_;
         FPolyS f;
         f.tau = tau;
         pointwise(f, s3, {LTS, LTA});
@@ -3364,7 +3364,6 @@ void Engine<T>::lsg_trial(double tau, double out[3], double* lqq) {
             wspec(WA), wspec(ls_wspec(0)), wspec(ls_wspec(1)), wspec(ls_wspec(2)), nsp, 1.0, tau, tau * tau, nullptr);
         launched("spec_poly", 4.0 * nsp * sizeof(cpx<T>), ev);
     } else {
-        ++ls_fft_trials_;
         FPolyS1 f;
         f.tau = tau;
         pointwise(f, s3, {LTS});
