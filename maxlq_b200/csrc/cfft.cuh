@@ -121,8 +121,9 @@ __device__ __forceinline__ cpx<T> cmul_s(cpx<T> a, cpx<T> w) {
 // before and which spend their time on FP64 twiddle loads and an integer
 // division per element: x inverse 986 -> 3800 GB/s, y forward 825 -> 3470, z
 // round trip 633 -> 1870 at 384^3 FP32, a CG iteration 58 -> 22 ms (mixed) and
-// at 192^3 7.8 -> 3.5 ms.  9 2^a would need a thread count of 3 2^j per line
-// and keeps the run-time kernels.
+// at 192^3 7.8 -> 3.5 ms.  9 2^a would take a last stage of radix 9 or 18 (3 x 3
+// with twiddles between the two), which is not written; it keeps the run-time
+// kernels.
 // ----------------------------------------------------------------------------
 template <int L, int E>
 struct CPlan {

@@ -110,11 +110,10 @@ class EngineBase {
     // up to 8 vector inner products; kinds 0 L2, 1 H_l, 2 div energy,
     // 3 curl energy sum |K x a|^2, 4 Laplacian energy sum |K|^4 |a|^2
     // (kinds 2-4 read only a)
-    // pairs' inner products; optionally ax_out <- ax_x + ax_a ax_y first, in
-    // the same pass (the pairs may name ax_out)
     void dots(const SpecDotPair* pairs, int np, double* out);
     // the same, left in the results (RS_IP ...) on the device; with ax_out,
-    // ax_out <- ax_x - alpha ax_y, alpha from the results (RS_CC)
+    // ax_out <- ax_x - alpha ax_y first, in the same pass (the pairs may name
+    // ax_out), alpha from the results (RS_CC)
     void dots_async(const SpecDotPair* pairs, int np, SVec* ax_out = nullptr, const SVec* ax_x = nullptr,
                     const SVec* ax_y = nullptr);
     // hilbert_leray of f1 and of f2 scaled by ||u||_q^{1-q} (||u||_q^q in
@@ -499,6 +498,10 @@ class Engine : public EngineBase {
     bool need_A() const { return P.q + MACH_EPSILON >= 4.0; }
     // even q (6 and 8): the coefficients of the trial's integrals where S(tau)
     // >= 0 at every point (at q = 6 the norm takes one transform per trial)
+    // The scheme is one of every even q; it ends at 8, the largest exponent of the
+    // configurations.  At q = 10 the setup would need |phi|^6 too, seven more
+    // coefficient fields (some 20 transforms, on the 21 of q = 8) against the 6
+    // or so that a trial there makes; neither was measured.
     bool lsg_poly_ok() const { return !use_e_u && (P.q == 6.0 || P.q == 8.0); }
     void lsg_poly_setup();
     bool lsg_poly_fetched_ = false;

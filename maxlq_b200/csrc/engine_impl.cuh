@@ -2466,9 +2466,9 @@ __global__ void __launch_bounds__(RED_THREADS, 4)
 template <typename T>
 __global__ void __launch_bounds__(RED_THREADS)
     ls_min_kernel(const T* __restrict__ s0, const T* __restrict__ s1, const T* __restrict__ s2, long npts, double tau,
-                  const double* __restrict__ taup, double* __restrict__ out) {
+                  double* __restrict__ out) {
     pdl_begin();
-    const T t = (T)(taup ? *taup : tau);
+    const T t = (T)tau;
     T m = T(1e30);
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < npts; i += (long)gridDim.x * blockDim.x)
         m = fmin(m, s0[i] + t * (s1[i] + t * s2[i]));
@@ -2995,7 +2995,7 @@ bool Engine<T>::ls_clamp_free(double tau) {
                 for (int a = 0; a < 3; ++a) sp[a] = phys(ls_phys(a));
             }
             cudaEvent_t ev = prof_mark();
-            launch_k(ls_min_kernel<T>, grid, RED_THREADS, 0, sp[0], sp[1], sp[2], npts, tau, nullptr, d_partials);
+            launch_k(ls_min_kernel<T>, grid, RED_THREADS, 0, sp[0], sp[1], sp[2], npts, tau, d_partials);
             launched("ls_min", 3.0 * npts * sizeof(T), ev);
             MLQ_CUDA(cudaMemcpyAsync(h.data(), d_partials, h.size() * sizeof(double), cudaMemcpyDeviceToHost, stream));
             MLQ_CUDA(cudaStreamSynchronize(stream));
