@@ -492,6 +492,8 @@ class Engine : public EngineBase {
     void lsg_setup(const SVec* u, const SVec* d, double tau0 = 0.0);
     void lsg_trial(double tau, double out[3], double* lqq);
     bool lsg_exact(double tau);
+    // for tau > 0, from the means of |u|^2, 2 u . d and |d|^2
+    static bool lsg_angle_ok(double s0, double s1, double s2) { return s1 >= -std::sqrt(s0 * s2); }
     // ||.||^2 of the power |.|^k of the S and A that the chain reads
     int power_sq(double k);
     // some power of R, the gradient or the norm is a product with A = P2(g^2)

@@ -3150,8 +3150,7 @@ template <typename T>
 bool Engine<T>::lsg_exact(double tau) {
     ls_poly_to_host();
     const cpx<T>* m = (const cpx<T>*)((const char*)h_ls_ + 896);
-    const double s0 = m[0].x, s1 = m[1].x, s2 = m[2].x;  // s1 = 2 <u, d>
-    return (tau < 0.0 ? -s1 : s1) >= -std::sqrt(s0 * s2);
+    return lsg_angle_ok(m[0].x, tau < 0.0 ? -m[1].x : m[1].x, m[2].x);
 }
 
 // The Parseval products of two polynomial spectra, by power of tau: one pass

@@ -96,13 +96,21 @@ class Solver : public SolverBase {
     bool lsg_ready = false;  // the same at q != 4
     // tau_near: a step the trials will visit the neighbourhood of (the
     // previous step in the CG loop), for the setup's clamp-free intervals
-    void ls_begin(const SVec* base, const SVec* dir, double tau_near = 0.0) {
+    // given: dir comes from the caller, not from a run, and may undo base; its
+    // angle is asked before the setup, which whole evaluations do not need
+    void ls_begin(const SVec* base, const SVec* dir, double tau_near = 0.0, bool given = false) {
         trials.clear();
         ls_ready = lsg_ready = false;
         if (e.ls_ok() && dir && e.ls_fits()) {
             e.ls_setup(base, dir, tau_near);
             ls_ready = true;
         } else if (e.lsg_ok() && dir) {
+            if (given) {
+                const SpecDotPair p[3] = {{base, base, 0}, {base, dir, 0}, {dir, dir, 0}};
+                double m[3];
+                e.dots(p, 3, m);
+                if (!e.lsg_angle_ok(m[0], 2.0 * m[1], m[2])) return;
+            }
             lsg_ready = in_search([&] {
                 if (!e.lsg_fits()) return false;
                 e.lsg_setup(base, dir, tau_near);
@@ -506,7 +514,7 @@ class Solver : public SolverBase {
     int mnbrak_host(const double* phi, const double* d, double tA0, double tB0, double br[2], int* flag) override {
         load(phi, tmp);
         load(d, c);
-        ls_begin(tmp, c, tB0);
+        ls_begin(tmp, c, tB0, true);
         *flag = 0;
         mnbrak(tmp, c, tA0, tB0, br, flag);
         trials.clear();
@@ -516,7 +524,7 @@ class Solver : public SolverBase {
     double brent_host(const double* phi, const double* d, const double br[2]) override {
         load(phi, tmp);
         load(d, c);
-        ls_begin(tmp, c, std::max(br[0], br[1]) * 0.381966);
+        ls_begin(tmp, c, std::max(br[0], br[1]) * 0.381966, true);
         const double x = brent(tmp, c, br, nullptr);
         trials.clear();
         started = false;

@@ -120,3 +120,19 @@ def test_bracket_along_the_full_gradient_in_mixed_precision(n, q, monkeypatch):
     assert f0 == f1
     n0, n1 = c0["line_search_trials_whole"], c1["line_search_trials_whole"]
     assert n1 > 0 and c1["line_search_trials_polynomial"] == c1["line_search_trials_transform"] == 0
+
+
+# and such a search takes no coefficient fields: 42 or more of a field's size
+@pytest.mark.parametrize("n,q", [(32, 6.0), (24, 3.0)])
+def test_whole_evaluations_need_no_search_fields(n, q):
+    with mlq.MaxLq(n, q, 1.0) as c:
+        u = c.rescaleLqNorm(c.seed_field(0, 2.0, n / 12))
+        d = c.divAvg_free(c.HilbertGradient(c.GradL2ForLq(u), 1.5 - 1.0 / q))
+        d *= np.sqrt((u * u).sum() / (d * d).sum())
+        c.calc_global_dLqdt_inclParts(u)
+        before = c.device_bytes
+        tb, flag = c.mnbrak(u, d, 0.0, 1.0)
+        assert flag == 0
+        c.brent(u, d, tb)
+        assert c.kernel_config()["line_search_trials_whole"] > 0
+        assert c.device_bytes - before < 30 * 8 * n**3
