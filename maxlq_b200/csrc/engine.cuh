@@ -480,7 +480,14 @@ class Engine : public EngineBase {
     // the same at the other exponents (and on the e_u branch): the setup
     // forms what is quadratic in tau, a trial transforms the products that
     // are not.  Resident mode only; MLQ_REUSE=0 evaluates R whole per trial.
-    bool lsg_ok() const { return !ls_ok() && !slab_ && reuse_on_; }
+    // Not in FP32 for q < 4 without unit vectors: |phi|^{q-4} then grows without
+    // bound where |phi|^2 is no more than its rounding, and with it what the
+    // separately rounded coefficients leave there.  At q = 3, 32^3, the trial
+    // values of 10 in 960 iterations were off by 2e-3 to 1e-2, with whole
+    // evaluations of 2.
+    bool lsg_ok() const {
+        return !ls_ok() && (sizeof(T) == 8 || use_e_u || P.q > 4.0) && !slab_ && reuse_on_;
+    }
     bool lsg_fits();
     void lsg_release();
     void lsg_give_up();

@@ -624,7 +624,7 @@ struct FLSE {
 // integrated against a field of the band, on which the dealias acts as the
 // identity: P2(A a4) against G, and P2(sum V^2) against a4.  a2 of the
 // reference is P2(A a4), or, with `direct`, the field given in A's place.
-// RAW: a4 is an undealiased power (0 < q - 4 < 2, or q < 4), so sum V^2 and a4
+// RAW: a4 is an undealiased power (0 < q - 4 < 2), so sum V^2 and a4
 // are outputs too.  inputs V_aj at 3a + j (9), p_a (3), u(3), d(3), a4, A, G_a (3)
 template <bool RAW>
 struct FLSTrial {

@@ -14,3 +14,14 @@ def test_trials_are_counted_by_how_they_are_formed(q, polynomial):
         k = c.kernel_config()
     assert (k["line_search_trials_polynomial"] > 0) == polynomial
     assert k["line_search_trials_polynomial"] + k["line_search_trials_transform"] > 0
+
+
+# FP32 at q < 4 without unit vectors: the power |phi|^{q-4} amplifies what separately rounded coefficients leave at small
+# |phi|
+def test_negative_powers_evaluate_whole_in_mixed_precision():
+    with mlq.MaxLq(32, 3.0, 1.0, precision="mixed", optim_tol=0.0, use_e_u_auto=0, use_e_u=0) as c:
+        c.state_load(c.seed_field(3, 2.0, 32 / 12))
+        c.state_iterate(3)
+        k = c.kernel_config()
+    assert k["line_search_trials_polynomial"] == k["line_search_trials_transform"] == 0
+    assert k["line_search_trials_whole"] > 0
