@@ -2584,7 +2584,7 @@ void Engine<T>::ls_qg_fields(const LsFields& lf, bool g_phys) {
     for (int a = 0; a < 3; ++a) {
         o[a].sym = SYM_INV_KSQ;
         o[a].phys_out = LP + a;
-        if (!slab_) {  // the next gradient's pressure source is a polynomial in tau of these
+        if (!slab_) {  // the next gradient's pressure source at q = 4 is a polynomial in tau of these
             o[a].spec = wspec(WLQ + a);
             o[a].spec_f64 = wf64<T>();
         }
